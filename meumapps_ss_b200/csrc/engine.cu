@@ -77,6 +77,28 @@ __global__ void __launch_bounds__(RED_THREADS) k_grad_energy(const DevConst* __r
   block_reduce_store(acc, 0, out + blockIdx.x);
 }
 
+// Q(k) of every k against the reference's rcond <= 1e-16 stop (ModElastic.f:187), for the
+// path whose z kernel only inverts (k_el_z)
+__global__ void __launch_bounds__(256) k_el_qcheck(const DevConst* __restrict__ Kp, int* err) {
+  const DevConst& K = *Kp;
+  for (int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < K.nk; id += (int64_t)gridDim.x * blockDim.x) {
+    if (id == 0) continue;
+    int kx, ky, kz;
+    kdecode(K, id, kx, ky, kz);
+    double a[3], b[3], Q[9];
+    kvec(K, kx, ky, kz, a, b);
+    build_q(K, a, b, Q);
+    set_err(err, invert3(Q, MEU_ERR_Q_SINGULAR));
+  }
+}
+// the six convergence sums from k_el_z's block partials, in a fixed order
+__global__ void __launch_bounds__(1024) k_el_zsum(const double* __restrict__ part, int nblk, double* out) {
+  const double* p = part + (int64_t)blockIdx.x * nblk;
+  double acc = 0;
+  for (int i = threadIdx.x; i < nblk; i += blockDim.x) acc += p[i];
+  block_reduce_store(acc, 0, out + blockIdx.x);
+}
+
 // the fluctuation spectrum has no k = 0 mode
 template <typename R>
 __global__ void k_zero_k0(cplx<R>* kc) {
@@ -382,6 +404,31 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
     };
     g_el_k = resident((const void*)k_el_k<R>);
     g_lan_k1 = resident((const void*)k_lan_k1<R>);
+    if (strain) {
+      // fused z kernel of the fixed point: supported lengths, symmetric stiffness (Q(k) is
+      // then symmetric; build_q's general form serves any other)
+      bool sym = true;
+      for (int i = 0; i < 6; ++i)
+        for (int j = 0; j < i; ++j) sym = sym && hK.c0m[i + j * 6] == hK.c0m[j + i * 6];
+      elz_blocks = sym ? el_z_blocks<R>(p.nz, p.ny * hK.nxh) : 0;
+      if (elz_blocks) {
+        elz_part = dalloc<double>(6 * (int64_t)elz_blocks);
+        int ex = 0;
+        double big = 0;
+        for (int i = 0; i < 36; ++i) big = std::max(big, std::fabs(hK.qcoef[i / 6][i % 6]));
+        std::frexp(big, &ex);
+        elz.qs = std::isfinite(big) && big > 0 ? std::ldexp(1.0, -ex) : 1.0;
+        for (int i = 0; i < 36; ++i) elz.q[i / 6][i % 6] = hK.qcoef[i / 6][i % 6] * elz.qs;
+        elz.scale = 1.0 / ((double)p.nx * p.ny * p.nz);
+        elz.wx = 6.283185307179586476925286766559 / (double)p.nx;
+        elz.wy = 6.283185307179586476925286766559 / (double)p.ny;
+        elz.nx = p.nx;
+        elz.ny = p.ny;
+        elz.nxh = hK.nxh;
+        elz.inner = p.ny * hK.nxh;
+        elz.ortho = ortho6(hK.c0m) ? 1 : 0;
+      }
+    }
     el_ortho_gen = ortho6(hK.c0m);
     for (int n = 0; n < p.numph; ++n) el_ortho_gen = el_ortho_gen && ortho6(p.sela[n]);
     g_elener = resident(el_ortho_gen ? (const void*)k_elener<R, true> : (const void*)k_elener<R>);
@@ -800,6 +847,13 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
     bool converged = false;
     std::vector<R*> out;
     for (int m = 0; m < 6; ++m) out.push_back(field(strain, m));
+    // y and x inverse of the six strain spectra after the fused z kernel
+    auto inverse_yx = [&](const std::vector<R*>& o) {
+      PtrList<R> b{};
+      for (int m = 0; m < 6; ++m) b.p[m] = o[m];
+      fft->pass_y<R>(specs(0, 6), 6, false, st);
+      fft->inverse_x<R>(specs(0, 6), b, 6, st);
+    };
     // spec(0..5) holds the strain spectrum of the last el_k and the real strain is not
     // formed yet: the next iteration runs its x passes and el_x as one kernel
     bool spec_pending = false;
@@ -807,11 +861,14 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
       niter += 1;
       total += 1;
       if (total > 100000) throw CudaError("elastic iteration runaway", MEU_ERR_NOT_CONVERGED);
+      // with the fused z kernel the spectra of an iteration have had their z inverse pass
       if (spec_pending) {
-        fft->inverse_cols<R>(specs(0, 6), 6, st);
+        if (elz_blocks) fft->pass_y<R>(specs(0, 6), 6, false, st);
+        else fft->inverse_cols<R>(specs(0, 6), 6, st);
         KLAUNCH("el_rows", 6.0 * 2 * nk * sizeof(C) + (double)V * n3 * sizeof(R),
                 el_rows_launch<R>(*fft, specs(0, 6), pphi, el_prop_r, el_ortho, cfac, d_err, st));
-        fft->forward_cols<R>(specs(0, 6), 6, st);
+        if (elz_blocks) fft->pass_y<R>(specs(0, 6), 6, true, st);
+        else fft->forward_cols<R>(specs(0, 6), 6, st);
         spec_pending = false;
       } else {
         if (hK.prop_moduli) {
@@ -820,16 +877,32 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
         } else
           KLAUNCH("el_x", (double)(V + 12) * n3 * sizeof(R),
                   (el_ortho_gen ? k_el_x<R, true> : k_el_x<R>)<<<gridr(), 256, 0, st>>>(dK, pphi, strain, xs, cfac, d_err));
-        std::vector<const R*> in;
-        for (int m = 0; m < 6; ++m) in.push_back(field(xs, m));
-        fwd_list(in, 0);
+        if (elz_blocks) {
+          PtrList<const R> in{};
+          for (int m = 0; m < 6; ++m) in.p[m] = field(xs, m);
+          fft->forward_x<R>(in, specs(0, 6), 6, st);
+          fft->pass_y<R>(specs(0, 6), 6, true, st);
+        } else {
+          std::vector<const R*> in;
+          for (int m = 0; m < 6; ++m) in.push_back(field(xs, m));
+          fwd_list(in, 0);
+        }
       }
-      KLAUNCH("el_k", 18.0 * nk * sizeof(C), k_el_k<R><<<g_el_k, RED_THREADS, 0, st>>>(dK, specs(0, 6), uk, partials, d_err));
-      if (el_fused_rows) spec_pending = true;
-      else inv_list(0, out);
-      finalize(Q_ERR0, 6);
+      if (elz_blocks) {
+        if (!elz_q_checked) KLAUNCH("el_qcheck", 0.0, k_el_qcheck<<<gridk(), 256, 0, st>>>(dK, d_err));
+        KLAUNCH("el_z", 18.0 * nk * sizeof(C), el_z_launch<R>(*fft, spec(0), uk, elz, elz_part, st));
+        KLAUNCH("finalize", 48.0 * elz_blocks, k_el_zsum<<<6, 1024, 0, st>>>(elz_part, elz_blocks, results + Q_ERR0));
+        if (el_fused_rows) spec_pending = true;
+        else inverse_yx(out);
+      } else {
+        KLAUNCH("el_k", 18.0 * nk * sizeof(C), k_el_k<R><<<g_el_k, RED_THREADS, 0, st>>>(dK, specs(0, 6), uk, partials, d_err));
+        if (el_fused_rows) spec_pending = true;
+        else inv_list(0, out);
+        finalize(Q_ERR0, 6);
+      }
       MEU_CUDA(cudaMemcpyAsync(h_results + Q_ERR0, results + Q_ERR0, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
       check_err();  // synchronises
+      elz_q_checked = elz_blocks > 0;
       double err[6];
       for (int q = 0; q < 6; ++q) err[q] = h_results[Q_ERR0 + q] * (double)n3;
       const double tol = P.el_tol;
@@ -857,7 +930,10 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
       }
       break;
     }
-    if (spec_pending) inv_list(0, out);
+    if (spec_pending) {
+      if (elz_blocks) inverse_yx(out);
+      else inv_list(0, out);
+    }
   }
   last_iters = total;
   const int eta2 = (P.model == MEU_MODEL_LANDAU && P.eig_coupling == MEU_EIG_ETA2) ? 1 : 0;

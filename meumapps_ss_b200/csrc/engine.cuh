@@ -46,6 +46,19 @@ struct ElenProp {
   int use[MEU_MAX_VAR];       // phase >= 2 and use_var: gets an energy share and a driving force
   int nvar;
 };
+// z-direction work of one elastic iteration in one pass (el_z.cuh): Q(k) of the matrix
+// ModElastic.f:119-158 as 6 x 6 coefficients on (a1^2, a2^2, a3^2, b2 b3, b1 b3, b1 b2),
+// scaled by the power of two qs (det Q then stays far from the range limits)
+struct ElzCoef {
+  double q[6][6], qs, scale, wx, wy;
+  int nx, ny, nxh, inner, ortho;
+};
+// blocks of the z kernel (each writes six partial sums); 0: no kernel for the length
+template <typename R>
+int el_z_blocks(int nz, int inner);
+// sp: six contiguous spectra; part: [6][el_z_blocks] partial sums of the convergence test
+template <typename R>
+void el_z_launch(const FFT3& f, cplx<R>* sp, cplx<R>* uk, const ElzCoef& E, double* part, cudaStream_t st);
 // x-direction work of one elastic iteration in one pass (el_rows.cu): x C2R of the six
 // strain spectra, polarisation, x R2C into the same spectra; row length nx/2 a power
 // of two in 32..512 (el_rows_ok)
@@ -309,6 +322,10 @@ class Engine : public EngineBase {
   bool el_ortho = false;              // stiffnesses with decoupled normal / shear blocks
   bool el_ortho_gen = false;          // general moduli: C0 and every phase's compliance in that pattern
   bool el_fused_rows = false;         // iterations run the x passes and el_x as one kernel
+  int elz_blocks = 0;                 // > 0: iterations run the z passes and the k-space work as one kernel
+  ElzCoef elz{};
+  double* elz_part = nullptr;         // its block partials [6][elz_blocks]
+  bool elz_q_checked = false;         // Q(k) tested by k_el_qcheck (it does not change in time)
   bool fused_warm = false;
   bool q_checked = false;  // Q(k) of the fused step tested (LS_QCHECK on its first step)
   bool theta_ready = false;  // sp holds theta^ of the current fields (written by the last step's PI)

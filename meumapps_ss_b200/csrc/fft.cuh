@@ -108,6 +108,72 @@ template <int S, typename C> struct Dft<8, S, C> {
   }
 };
 
+// 6 = 2 x 3 and 12 = 3 x 4 by the Good-Thomas index maps (coprime factors: no twiddles);
+// 9 = 3 x 3 with the twiddles W9^(bc).  Used by the mixed plans of lengths with factors 3.
+template <int S, typename C> struct Dft<6, S, C> {
+  static __device__ __forceinline__ void run(C* x) {
+    // n = 3 n1 + 2 n2 (mod 6), k = 3 k1 + 4 k2 (mod 6)
+    C a[3] = {x[0], x[2], x[4]}, b[3] = {x[3], x[5], x[1]};
+    Dft<3, S, C>::run(a);
+    Dft<3, S, C>::run(b);
+    x[0] = cadd(a[0], b[0]);
+    x[3] = csub(a[0], b[0]);
+    x[4] = cadd(a[1], b[1]);
+    x[1] = csub(a[1], b[1]);
+    x[2] = cadd(a[2], b[2]);
+    x[5] = csub(a[2], b[2]);
+  }
+};
+template <int S, typename C> struct Dft<12, S, C> {
+  static __device__ __forceinline__ void run(C* x) {
+    // n = 4 n1 + 3 n2 (mod 12), k = 4 k1 + 9 k2 (mod 12)
+    C t[3][4];
+#pragma unroll
+    for (int n1 = 0; n1 < 3; ++n1) {
+#pragma unroll
+      for (int n2 = 0; n2 < 4; ++n2) t[n1][n2] = x[(4 * n1 + 3 * n2) % 12];
+      Dft<4, S, C>::run(t[n1]);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < 4; ++k2) {
+      C v[3] = {t[0][k2], t[1][k2], t[2][k2]};
+      Dft<3, S, C>::run(v);
+#pragma unroll
+      for (int k1 = 0; k1 < 3; ++k1) x[(4 * k1 + 9 * k2) % 12] = v[k1];
+    }
+  }
+};
+template <int S, typename C> struct Dft<9, S, C> {
+  static __device__ __forceinline__ void run(C* x) {
+    using R = decltype(x[0].x);
+    // cos and sin of 2 pi k / 9, k = 1, 2, 4
+    const R c1 = (R)0.76604444311897803520, s1 = (R)0.64278760968653932632;
+    const R c2 = (R)0.17364817766693034885, s2 = (R)0.98480775301220805937;
+    const R c4 = (R)-0.93969262078590838405, s4 = (R)0.34202014332566873304;
+    const R sg = (R)S;
+    auto w = [](C v, R cr, R ci) { return mk(v.x * cr - v.y * ci, v.x * ci + v.y * cr); };
+    C t[9];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      C v[3] = {x[b], x[3 + b], x[6 + b]};
+      Dft<3, S, C>::run(v);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) t[3 * b + c] = v[c];
+    }
+    t[4] = w(t[4], c1, sg * s1);  // b=1 c=1
+    t[5] = w(t[5], c2, sg * s2);  // b=1 c=2
+    t[7] = w(t[7], c2, sg * s2);  // b=2 c=1
+    t[8] = w(t[8], c4, sg * s4);  // b=2 c=2
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      C v[3] = {t[c], t[3 + c], t[6 + c]};
+      Dft<3, S, C>::run(v);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) x[c + 3 * d] = v[d];
+    }
+  }
+};
+
 // 16 points as 4 x 4: radix-4 over a of x[4a+b], twiddle W16^(b c), radix-4 over b
 // (y[c + 4d] = sum_b W4^(bd) W16^(bc) sum_a W4^(ac) x[4a+b]).  Constants in the field
 // precision (the fused transforms only).

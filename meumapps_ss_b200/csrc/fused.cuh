@@ -31,6 +31,9 @@ struct RPlan {
 //   pv 1: radix 4 first (128 = 4*4*4*2), then at most one 2, then 3s;
 //   pv 2: radix 16 first, then 8s, 4s, at most one 2, 3s (128 = 16*8: one
 //         shared-memory pass fewer, more registers per butterfly).
+// pv 3 is the generic path's plan of any supported 2^a 3^b length: as few stages as radices
+// up to 16 allow (every length up to 256 except 162 and 216 in two stages, so a line makes
+// one shared-memory round trip), 6, 9 and 12 taking the factors 3.
 __host__ __device__ constexpr int twos(int n) {
   int k = 0;
   while (n > 0 && n % 2 == 0) { n /= 2; ++k; }
@@ -39,6 +42,20 @@ __host__ __device__ constexpr int twos(int n) {
 __host__ __device__ constexpr RPlan rplan(int L, int pv = 0) {
   RPlan p{0, {1, 1, 1, 1, 1, 1, 1, 1}};
   int n = L;
+  if (pv == 3) {
+    const int tab[][4] = {{12, 4, 3, 1},  {16, 4, 4, 1},   {18, 6, 3, 1},   {24, 6, 4, 1},  {27, 9, 3, 1},
+                          {32, 8, 4, 1},  {36, 6, 6, 1},   {48, 8, 6, 1},   {54, 9, 6, 1},  {64, 8, 8, 1},
+                          {72, 9, 8, 1},  {81, 9, 9, 1},   {96, 12, 8, 1},  {108, 12, 9, 1}, {128, 16, 8, 1},
+                          {144, 12, 12, 1}, {162, 9, 6, 3}, {192, 16, 12, 1}, {216, 6, 6, 6}, {256, 16, 16, 1},
+                          {288, 8, 6, 6}, {324, 9, 6, 6},  {384, 8, 8, 6},  {432, 9, 8, 6}, {512, 8, 8, 8}};
+    for (const auto& e : tab)
+      if (e[0] == L) {
+        for (int i = 1; i < 4; ++i)
+          if (e[i] > 1) p.r[p.ns++] = e[i];
+        return p;
+      }
+    return p;  // no plan: ns = 0
+  }
   if (pv == 2) {
     while (n % 16 == 0) { p.r[p.ns++] = 16; n /= 16; }
     while (n % 8 == 0) { p.r[p.ns++] = 8; n /= 8; }
