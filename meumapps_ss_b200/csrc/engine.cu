@@ -140,16 +140,18 @@ __global__ void k_convert_in(const double* __restrict__ src, R* __restrict__ dst
 }
 // engineering strain from the 9 gradients grad_j_ui (data_save order (j-1)*3+(i-1))
 // gu holds nv voxels of each gradient back to back; strain is offset to the chunk
+// scale: 1, or 1/nx for the row spectra (whose x C2R is unscaled)
 template <typename R>
-__global__ void k_grads_to_strain(const double* __restrict__ gu, R* __restrict__ strain, int64_t nv, int64_t n3) {
+__global__ void k_grads_to_strain(const double* __restrict__ gu, R* __restrict__ strain, int64_t nv, int64_t n3,
+                                  double scale) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (int64_t)gridDim.x * blockDim.x) {
     auto G = [&](int ui, int dj) { return gu[(int64_t)((dj - 1) * 3 + (ui - 1)) * nv + i]; };
-    strain[0 * n3 + i] = (R)G(1, 1);
-    strain[1 * n3 + i] = (R)G(2, 2);
-    strain[2 * n3 + i] = (R)G(3, 3);
-    strain[3 * n3 + i] = (R)(G(3, 2) + G(2, 3));
-    strain[4 * n3 + i] = (R)(G(3, 1) + G(1, 3));
-    strain[5 * n3 + i] = (R)(G(2, 1) + G(1, 2));
+    strain[0 * n3 + i] = (R)(G(1, 1) * scale);
+    strain[1 * n3 + i] = (R)(G(2, 2) * scale);
+    strain[2 * n3 + i] = (R)(G(3, 3) * scale);
+    strain[3 * n3 + i] = (R)((G(3, 2) + G(2, 3)) * scale);
+    strain[4 * n3 + i] = (R)((G(3, 1) + G(1, 3)) * scale);
+    strain[5 * n3 + i] = (R)((G(2, 1) + G(1, 2)) * scale);
   }
 }
 // u^ -> [u_i^ (3), kf_j u_i^ (9)] in data_save order
@@ -302,9 +304,38 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
     NWR = 2 * V + 1;
     NS = 2 * V + 2;
   }
-  if (elast && het) {
-    strain = dalloc<R>(6 * n3);
-    xs = dalloc<R>(6 * n3);
+  el_ortho_gen = ortho6(hK.c0m);
+  for (int n = 0; n < p.numph; ++n) el_ortho_gen = el_ortho_gen && ortho6(p.sela[n]);
+  el_state = elast && het;
+  // the row kernels: their lengths, proportional moduli or general ones with decoupled normal
+  // and shear parts; anything else keeps the real strain and el_x
+  el_fused_rows = el_state && el_rows_ok(p.nx) && (hK.prop_moduli || el_ortho_gen);
+  if (el_state) {
+    if (el_fused_rows) {
+      es = dalloc<C>(6 * nk);
+      tw_nx = dalloc<C>(p.nx);
+      std::vector<C> tw(p.nx);
+      fft_twiddles(p.nx, sizeof(R) == 8, tw.data());
+      MEU_CUDA(cudaMemcpy(tw_nx, tw.data(), sizeof(C) * p.nx, cudaMemcpyHostToDevice));
+      for (int i = 0; i < 36; ++i) {
+        el_gen.c0[i] = hK.c0m[i];
+        for (int n = 0; n < p.numph; ++n) el_gen.s[n][i] = p.sela[n][i];
+      }
+      for (int m = 0; m < 6; ++m) el_gen.ebar[m] = hK.ebar_eng[m];
+      for (int v = 0; v < V; ++v) {
+        el_gen.phase[v] = hK.var_phase[v] - 1;
+        for (int m = 0; m < 6; ++m) el_gen.ep[v][m] = hK.eps_eng[v][m];
+      }
+      el_gen.nvar = V;
+      el_gen.numph = p.numph;
+      for (int n = 1; n < p.numph; ++n) {
+        el_gen.lo[n] = hK.ph_lo[n + 1];
+        el_gen.hi[n] = hK.ph_hi[n + 1];
+      }
+    } else {
+      strain = dalloc<R>(6 * n3);
+      xs = dalloc<R>(6 * n3);
+    }
     uk = dalloc<C>(3 * nk);
     NS = std::max(NS, V + 6);
   }
@@ -390,6 +421,7 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
   if (noise) MEU_CUDA(cudaMemset(noise, 0, sizeof(R) * V * n3));
   MEU_CUDA(cudaMemset(el_en, 0, sizeof(R) * n3));
   if (strain) MEU_CUDA(cudaMemset(strain, 0, sizeof(R) * 6 * n3));
+  if (es) MEU_CUDA(cudaMemset(es, 0, sizeof(C) * 6 * nk));
   if (uk) MEU_CUDA(cudaMemset(uk, 0, sizeof(C) * 3 * nk));
   stage_elems = std::min<int64_t>(n3 * std::max(std::max(V, E), 1), (int64_t)32 << 20);
   stage = dalloc<double>(stage_elems);
@@ -404,7 +436,7 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
     };
     g_el_k = resident((const void*)k_el_k<R>);
     g_lan_k1 = resident((const void*)k_lan_k1<R>);
-    if (strain) {
+    if (el_state) {
       // fused z kernel of the fixed point: supported lengths, symmetric stiffness (Q(k) is
       // then symmetric; build_q's general form serves any other)
       bool sym = true;
@@ -429,8 +461,6 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
         elz.ortho = ortho6(hK.c0m) ? 1 : 0;
       }
     }
-    el_ortho_gen = ortho6(hK.c0m);
-    for (int n = 0; n < p.numph; ++n) el_ortho_gen = el_ortho_gen && ortho6(p.sela[n]);
     g_elener = resident(el_ortho_gen ? (const void*)k_elener<R, true> : (const void*)k_elener<R>);
     if (hK.prop_moduli) {
       ElxProp& X = el_prop;
@@ -446,6 +476,8 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
         X.inc[v] = n >= 2 ? 1.0 : 0.0;
       }
       X.nvar = V;
+      const bool ortho = ortho6(hK.c0m) && ortho6(p.cela[0]) && ortho6(p.sela[0]);
+      X.ortho = ortho ? 1 : 0;
       el_prop_r.assign(X);
       ElenProp& Y = en_prop;
       for (int i = 0; i < 36; ++i) {
@@ -460,9 +492,7 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
         Y.use[v] = (n >= 2 && hK.use_var[v]) ? 1 : 0;
       }
       Y.nvar = V;
-      const bool ortho = ortho6(hK.c0m) && ortho6(p.cela[0]) && ortho6(p.sela[0]);
-      el_ortho = ortho;
-      el_fused_rows = el_rows_ok(p.nx);
+      Y.ortho = X.ortho;
       // 16-byte tile copies when every field starts on a 16-byte boundary
       const bool vec = n3 % (16 / (int64_t)sizeof(R)) == 0;
       fn_el_x = ortho ? (vec ? k_el_x_prop<R, true, true> : k_el_x_prop<R, true, false>)
@@ -616,7 +646,7 @@ void Engine<R>::check_err() {
 template <typename R>
 void Engine<R>::finalize(int q0, int nq, double* out, const int* nbs) {
   NbList nb;
-  for (int q = 0; q < nq; ++q) nb.nb[q] = nbs ? nbs[q] : RED_BLOCKS;
+  for (int q = 0; q < nq; ++q) nb.nb[q] = nbs ? nbs[q] : (q0 + q == Q_ELEN && el_fused_rows) ? PSTRIDE : RED_BLOCKS;
   KLAUNCH("finalize", 8.0 * nq * RED_BLOCKS,
           k_finalize<<<nq, 256, 0, st>>>(partials + (int64_t)q0 * PSTRIDE, nb, d_ops + q0, out ? out : results + q0));
 }
@@ -680,7 +710,7 @@ void Engine<R>::set_fields(const double* cons, const double* phi_in, const doubl
       KLAUNCH("zero_k0", 16.0, k_zero_k0<R><<<1, 32, 0, st>>>(kc));
     }
   }
-  if (strain) {
+  if (el_state) {
     if (ustate) {
       // u (3 x n3) -> u^ ; grads (9 x n3) -> engineering strain
       for (int i = 0; i < 3; ++i) {
@@ -696,18 +726,29 @@ void Engine<R>::set_fields(const double* cons, const double* phi_in, const doubl
         b.p[0] = uk + (int64_t)i * nk;
         fft->forward<R>(a, b, 1, st);
       }
-      // the 9 gradients, chunked through the staging buffer
+      // the 9 gradients, chunked through the staging buffer; the row path transforms the strain
+      // to its spectra (a temporary field: restarts only)
+      R* sd = strain;
+      if (el_fused_rows) MEU_CUDA(cudaMalloc((void**)&sd, sizeof(R) * 6 * (size_t)n3));
+      std::unique_ptr<R, void (*)(R*)> own(el_fused_rows ? sd : nullptr, [](R* q) { cudaFree(q); });
       const int64_t chunk = std::max<int64_t>(stage_elems / 9, 1);
       for (int64_t v0 = 0; v0 < n3; v0 += chunk) {
         const int64_t nv = std::min(chunk, n3 - v0);
         for (int g = 0; g < 9; ++g)
           MEU_CUDA(cudaMemcpyAsync(stage + (int64_t)g * nv, ustate + (int64_t)(3 + g) * n3 + v0, sizeof(double) * nv,
                                    cudaMemcpyHostToDevice, st));
-        KLAUNCH("grads_to_strain", (double)nv * (9 * 8 + 6 * sizeof(R)), k_grads_to_strain<R><<<grid_for(nv, 256), 256, 0, st>>>(stage, strain + v0, nv, n3));
+        KLAUNCH("grads_to_strain", (double)nv * (9 * 8 + 6 * sizeof(R)), k_grads_to_strain<R><<<grid_for(nv, 256), 256, 0, st>>>(stage, sd + v0, nv, n3, el_fused_rows ? 1.0 / P.nx : 1.0));
+      }
+      if (el_fused_rows) {
+        PtrList<const R> a{};
+        for (int m = 0; m < 6; ++m) a.p[m] = sd + (int64_t)m * n3;
+        fft->forward_x<R>(a, es_list(), 6, st);
+        MEU_CUDA(cudaStreamSynchronize(st));  // sd is freed here
       }
       el_ready = true;
     } else {
-      MEU_CUDA(cudaMemsetAsync(strain, 0, sizeof(R) * 6 * n3, st));
+      if (es) MEU_CUDA(cudaMemsetAsync(es, 0, sizeof(C) * 6 * nk, st));
+      else MEU_CUDA(cudaMemsetAsync(strain, 0, sizeof(R) * 6 * n3, st));
       MEU_CUDA(cudaMemsetAsync(uk, 0, sizeof(C) * 3 * nk, st));
       el_ready = false;
     }
@@ -830,14 +871,19 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
   // enters later without an uploaded state starts from u = 0 like the reference.
   const bool do_zeroth = zeroth_only || step == P.elastep0;
   (void)first;
+  std::vector<R*> out;  // real strain (not on the row path)
+  if (!el_fused_rows)
+    for (int m = 0; m < 6; ++m) out.push_back(field(strain, m));
+  // the six spectra of an iteration: the row path works in place on its state
+  const PtrList<C> S6 = el_fused_rows ? es_list() : specs(0, 6);
   if (do_zeroth) {
     std::vector<const R*> in;
     for (int v = 0; v < V; ++v) in.push_back(field(pphi, v));
     fwd_list(in, 0);
-    KLAUNCH("el_zeroth", (double)(V + 9) * nk * sizeof(C), k_el_zeroth<R><<<gridk(), 256, 0, st>>>(dK, specs(0, V), V, uk, specs(V, 6), d_err));
-    std::vector<R*> out;
-    for (int m = 0; m < 6; ++m) out.push_back(field(strain, m));
-    inv_list(V, out);
+    KLAUNCH("el_zeroth", (double)(V + 9) * nk * sizeof(C),
+            k_el_zeroth<R><<<gridk(), 256, 0, st>>>(dK, specs(0, V), V, uk, el_fused_rows ? S6 : specs(V, 6), d_err));
+    if (el_fused_rows) fft->inverse_cols<R>(S6, 6, st);
+    else inv_list(V, out);
   }
   el_ready = true;
   int total = 0;
@@ -845,31 +891,18 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
     double newfac = 0.5, cfac = 1.0, err_old[6] = {0, 0, 0, 0, 0, 0};
     int niter = 0;
     bool converged = false;
-    std::vector<R*> out;
-    for (int m = 0; m < 6; ++m) out.push_back(field(strain, m));
-    // y and x inverse of the six strain spectra after the fused z kernel
-    auto inverse_yx = [&](const std::vector<R*>& o) {
-      PtrList<R> b{};
-      for (int m = 0; m < 6; ++m) b.p[m] = o[m];
-      fft->pass_y<R>(specs(0, 6), 6, false, st);
-      fft->inverse_x<R>(specs(0, 6), b, 6, st);
-    };
-    // spec(0..5) holds the strain spectrum of the last el_k and the real strain is not
-    // formed yet: the next iteration runs its x passes and el_x as one kernel
-    bool spec_pending = false;
     for (;;) {
       niter += 1;
       total += 1;
       if (total > 100000) throw CudaError("elastic iteration runaway", MEU_ERR_NOT_CONVERGED);
-      // with the fused z kernel the spectra of an iteration have had their z inverse pass
-      if (spec_pending) {
-        if (elz_blocks) fft->pass_y<R>(specs(0, 6), 6, false, st);
-        else fft->inverse_cols<R>(specs(0, 6), 6, st);
-        KLAUNCH("el_rows", 6.0 * 2 * nk * sizeof(C) + (double)V * n3 * sizeof(R),
-                el_rows_launch<R>(*fft, specs(0, 6), pphi, el_prop_r, el_ortho, cfac, d_err, st));
-        if (elz_blocks) fft->pass_y<R>(specs(0, 6), 6, true, st);
-        else fft->forward_cols<R>(specs(0, 6), 6, st);
-        spec_pending = false;
+      // ---- polarisation and its x transform
+      if (el_fused_rows) {
+        // the first iteration's polarisation in FP64 whatever the fields' precision
+        KLAUNCH("el_rows", 6.0 * 2 * nk * sizeof(C) + (double)V * n3 * sizeof(R), {
+          const ElRowsArgs<R> ra = rows_args();
+          if (!el_rows_a<R>(ra, rows_coef(), cfac, total == 1) && !el_rows_b<R>(ra, rows_coef(), cfac, total == 1))
+            throw CudaError("internal: fused elastic rows for an unsupported length", MEU_ERR_UNSUPPORTED);
+        });
       } else {
         if (hK.prop_moduli) {
           KLAUNCH("el_x", (double)(V + 12) * n3 * sizeof(R),
@@ -877,28 +910,27 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
         } else
           KLAUNCH("el_x", (double)(V + 12) * n3 * sizeof(R),
                   (el_ortho_gen ? k_el_x<R, true> : k_el_x<R>)<<<gridr(), 256, 0, st>>>(dK, pphi, strain, xs, cfac, d_err));
-        if (elz_blocks) {
-          PtrList<const R> in{};
-          for (int m = 0; m < 6; ++m) in.p[m] = field(xs, m);
-          fft->forward_x<R>(in, specs(0, 6), 6, st);
-          fft->pass_y<R>(specs(0, 6), 6, true, st);
-        } else {
-          std::vector<const R*> in;
-          for (int m = 0; m < 6; ++m) in.push_back(field(xs, m));
-          fwd_list(in, 0);
-        }
+        PtrList<const R> in{};
+        for (int m = 0; m < 6; ++m) in.p[m] = field(xs, m);
+        fft->forward_x<R>(in, S6, 6, st);
       }
+      // ---- y, k-space, y
+      fft->pass_y<R>(S6, 6, true, st);
       if (elz_blocks) {
         if (!elz_q_checked) KLAUNCH("el_qcheck", 0.0, k_el_qcheck<<<gridk(), 256, 0, st>>>(dK, d_err));
-        KLAUNCH("el_z", 18.0 * nk * sizeof(C), el_z_launch<R>(*fft, spec(0), uk, elz, elz_part, st));
+        KLAUNCH("el_z", 18.0 * nk * sizeof(C), el_z_launch<R>(*fft, S6.p[0], uk, elz, elz_part, st));
         KLAUNCH("finalize", 48.0 * elz_blocks, k_el_zsum<<<6, 1024, 0, st>>>(elz_part, elz_blocks, results + Q_ERR0));
-        if (el_fused_rows) spec_pending = true;
-        else inverse_yx(out);
       } else {
-        KLAUNCH("el_k", 18.0 * nk * sizeof(C), k_el_k<R><<<g_el_k, RED_THREADS, 0, st>>>(dK, specs(0, 6), uk, partials, d_err));
-        if (el_fused_rows) spec_pending = true;
-        else inv_list(0, out);
+        fft->pass_z<R>(S6, 6, true, st);
+        KLAUNCH("el_k", 18.0 * nk * sizeof(C), k_el_k<R><<<g_el_k, RED_THREADS, 0, st>>>(dK, S6, uk, partials, d_err));
+        fft->pass_z<R>(S6, 6, false, st);
         finalize(Q_ERR0, 6);
+      }
+      fft->pass_y<R>(S6, 6, false, st);
+      if (!el_fused_rows) {
+        PtrList<R> o{};
+        for (int m = 0; m < 6; ++m) o.p[m] = out[m];
+        fft->inverse_x<R>(S6, o, 6, st);
       }
       MEU_CUDA(cudaMemcpyAsync(h_results + Q_ERR0, results + Q_ERR0, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
       check_err();  // synchronises
@@ -930,22 +962,24 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
       }
       break;
     }
-    if (spec_pending) {
-      if (elz_blocks) inverse_yx(out);
-      else inv_list(0, out);
-    }
   }
   last_iters = total;
   const int eta2 = (P.model == MEU_MODEL_LANDAU && P.eig_coupling == MEU_EIG_ETA2) ? 1 : 0;
-  if (hK.prop_moduli) {
+  if (el_fused_rows) {
+    KLAUNCH("elener", 6.0 * nk * sizeof(C) + (double)(2 * V + 1 + V) * n3 * sizeof(R), {
+      const ElRowsArgs<R> ra = rows_args();
+      if (!el_ener_a<R>(ra, rows_coef(), ph_for_ppr, dK, el_en, elg, mode, eta2, partials) &&
+          !el_ener_b<R>(ra, rows_coef(), ph_for_ppr, dK, el_en, elg, mode, eta2, partials))
+        throw CudaError("internal: elastic energy rows for an unsupported length", MEU_ERR_UNSUPPORTED);
+    });
+  } else if (hK.prop_moduli) {
     KLAUNCH("elener", (double)(2 * V + 6 + 1 + V) * n3 * sizeof(R),
             fn_elener<<<g_elener, PF_TILE, sm_elener, st>>>(en_prop, (int64_t)n3, ph_for_ppr, pphi, strain, el_en, elg,
                                                             mode, eta2, partials, d_err));
   } else
     KLAUNCH("elener", (double)(2 * V + 6 + 1 + V) * n3 * sizeof(R),
-            (el_ortho_gen ? k_elener<R, true> : k_elener<R>)<<<g_elener, RED_THREADS, 0, st>>>(dK, ph_for_ppr, pphi, strain, el_en, elg, mode,
-                                                  (P.model == MEU_MODEL_LANDAU && P.eig_coupling == MEU_EIG_ETA2) ? 1 : 0,
-                                                  partials, d_err));
+            (el_ortho_gen ? k_elener<R, true> : k_elener<R>)<<<g_elener, RED_THREADS, 0, st>>>(
+                dK, ph_for_ppr, pphi, strain, el_en, elg, mode, eta2, partials, d_err));
 }
 
 // ------------------------------------------------------------------- KKS step

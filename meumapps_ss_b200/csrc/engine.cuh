@@ -21,7 +21,7 @@ struct ElxCoef {
   W ep[MEU_MAX_VAR][6];
   W av[MEU_MAX_VAR];   // alpha of the variant's phase, 0 for phase-1 variants
   W inc[MEU_MAX_VAR];  // 1 when the variant counts toward sum P (phase >= 2)
-  int nvar;
+  int nvar, ortho;     // ortho: c0 and c1 have decoupled normal / shear parts (mv6<true>)
   template <typename U>
   void assign(const ElxCoef<U>& o) {
     for (int i = 0; i < 36; ++i) {
@@ -35,6 +35,7 @@ struct ElxCoef {
       inc[v] = (W)o.inc[v];
     }
     nvar = o.nvar;
+    ortho = o.ortho;
   }
 };
 using ElxProp = ElxCoef<double>;
@@ -44,7 +45,13 @@ struct ElenProp {
   double tp[MEU_MAX_VAR][6];  // trans_ppt (tensor shear)
   double av[MEU_MAX_VAR];     // alpha of the variant's phase, 0 for phase-1 variants
   int use[MEU_MAX_VAR];       // phase >= 2 and use_var: gets an energy share and a driving force
-  int nvar;
+  int nvar, ortho;
+};
+// general moduli with decoupled normal and shear parts (c0 and every compliance), by value to
+// the row kernels: s[n] the compliance of phase n + 1, phase[v] >= 1 the variant's index in s
+struct ElxGen {
+  double c0[36], s[MEU_MAX_PH][36], ep[MEU_MAX_VAR][6], ebar[6];
+  int phase[MEU_MAX_VAR], lo[MEU_MAX_PH], hi[MEU_MAX_PH], nvar, numph;  // [lo, hi): variants of phase n + 1
 };
 // z-direction work of one elastic iteration in one pass (el_z.cuh): Q(k) of the matrix
 // ModElastic.f:119-158 as 6 x 6 coefficients on (a1^2, a2^2, a3^2, b2 b3, b1 b3, b1 b2),
@@ -59,13 +66,42 @@ int el_z_blocks(int nz, int inner);
 // sp: six contiguous spectra; part: [6][el_z_blocks] partial sums of the convergence test
 template <typename R>
 void el_z_launch(const FFT3& f, cplx<R>* sp, cplx<R>* uk, const ElzCoef& E, double* part, cudaStream_t st);
-// x-direction work of one elastic iteration in one pass (el_rows.cu): x C2R of the six
-// strain spectra, polarisation, x R2C into the same spectra; row length nx/2 a power
-// of two in 32..512 (el_rows_ok)
-bool el_rows_ok(int nx);
+// x-direction work of one elastic iteration in one pass, and elener on the same row spectra
+// (el_rows.cuh): sp the six row spectra, nk apart; tw: exp(-2 pi i n / nx), n < nx
 template <typename R>
-void el_rows_launch(const FFT3& f, const PtrList<cplx<R>>& sp, const R* pphi, const ElxCoef<R>& E, bool ortho,
-                    double cfac, int* err, cudaStream_t st);
+struct ElRowsArgs {
+  cplx<R>* sp;
+  const R* pphi;
+  const void* tw;
+  int64_t nk, n3, nrows;
+  int nx;
+  int* err;
+  cudaStream_t st;
+};
+template <typename R>
+struct ElRowsCoef {
+  bool prop;                // proportional moduli: pr / p64 / en, else gen
+  const ElxCoef<R>* pr;     // in the field precision
+  const ElxProp* p64;
+  const ElenProp* en;
+  const ElxGen* gen;
+};
+// false: no kernel for nx (a: up to 128, b: longer).  fp64: the polarisation in FP64.
+template <typename R>
+bool el_rows_a(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, double cfac, bool fp64);
+template <typename R>
+bool el_rows_b(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, double cfac, bool fp64);
+template <typename R>
+bool el_ener_a(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, const R* phi, const DevConst* K, R* el_en, R* elg,
+               int mode, int eta2, double* partials);
+template <typename R>
+bool el_ener_b(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, const R* phi, const DevConst* K, R* el_en, R* elg,
+               int mode, int eta2, double* partials);
+inline bool el_rows_ok(int nx) {
+  for (int n : {16, 24, 32, 36, 48, 54, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 512, 1024})
+    if (nx == n) return true;
+  return false;
+}
 }  // namespace meu
 
 namespace meu {
@@ -319,9 +355,23 @@ class Engine : public EngineBase {
   void (*fn_el_x)(ElxProp, int64_t, const R*, const R*, R*, double, int*) = nullptr;
   void (*fn_elener)(ElenProp, int64_t, const R*, const R*, const R*, R*, R*, int, int, double*, int*) = nullptr;
   size_t sm_el_x = 0, sm_elener = 0;  // their dynamic shared memory (prefetch tiles)
-  bool el_ortho = false;              // stiffnesses with decoupled normal / shear blocks
   bool el_ortho_gen = false;          // general moduli: C0 and every phase's compliance in that pattern
-  bool el_fused_rows = false;         // iterations run the x passes and el_x as one kernel
+  // iterations run the x direction as one kernel on the row spectra es (six, nk apart), which
+  // replace the real strain and polarisation fields
+  bool el_fused_rows = false;
+  bool el_state = false;              // heterogeneous elasticity keeps a state between steps
+  C* es = nullptr;
+  C* tw_nx = nullptr;                 // exp(-2 pi i n / nx), n < nx
+  ElxGen el_gen{};
+  ElRowsArgs<R> rows_args() const {
+    return {es, pphi, tw_nx, nk, n3, (int64_t)P.ny * P.nz, P.nx, d_err, st};
+  }
+  ElRowsCoef<R> rows_coef() const { return {hK.prop_moduli != 0, &el_prop_r, &el_prop, &en_prop, &el_gen}; }
+  PtrList<C> es_list() const {
+    PtrList<C> l{};
+    for (int m = 0; m < 6; ++m) l.p[m] = es + (int64_t)m * nk;
+    return l;
+  }
   int elz_blocks = 0;                 // > 0: iterations run the z passes and the k-space work as one kernel
   ElzCoef elz{};
   double* elz_part = nullptr;         // its block partials [6][elz_blocks]

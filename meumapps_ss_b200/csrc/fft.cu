@@ -58,6 +58,15 @@ static void twiddle(int n, int L, long double& c, long double& s) {
   s = sinl(a);
 }
 
+void fft_twiddles(int L, bool fp64, void* host) {
+  for (int n = 0; n < L; ++n) {
+    long double c, s;
+    twiddle(n, L, c, s);
+    if (fp64) ((double2*)host)[n] = make_double2((double)c, (double)s);
+    else ((float2*)host)[n] = make_float2((float)(double)c, (float)(double)s);
+  }
+}
+
 size_t FFT3::table_bytes(int nx, int ny, int nz, bool fp64) {
   const size_t csz = fp64 ? sizeof(double2) : sizeof(float2);
   const int K = 1;

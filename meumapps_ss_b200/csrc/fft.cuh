@@ -345,5 +345,7 @@ class FFT3 {
 };
 
 bool fft_size_ok(int n, bool is_x);
+// exp(-2 pi i n / L), n < L, correctly rounded (host; float2 or double2)
+void fft_twiddles(int L, bool fp64, void* host);
 
 }  // namespace meu

@@ -34,6 +34,8 @@ struct RPlan {
 // pv 3 is the generic path's plan of any supported 2^a 3^b length: as few stages as radices
 // up to 16 allow (every length up to 256 except 162 and 216 in two stages, so a line makes
 // one shared-memory round trip), 6, 9 and 12 taking the factors 3.
+// pv 4 ends in a radix of 2 or 3: the plan of the elastic row kernels, whose last stage holds
+// the butterflies of six lines in registers.
 __host__ __device__ constexpr int twos(int n) {
   int k = 0;
   while (n > 0 && n % 2 == 0) { n /= 2; ++k; }
@@ -42,6 +44,21 @@ __host__ __device__ constexpr int twos(int n) {
 __host__ __device__ constexpr RPlan rplan(int L, int pv = 0) {
   RPlan p{0, {1, 1, 1, 1, 1, 1, 1, 1}};
   int n = L;
+  if (pv == 4) {
+    const int tab[][5] = {{16, 8, 2, 1, 1},    {24, 8, 3, 1, 1},   {32, 16, 2, 1, 1},  {36, 12, 3, 1, 1},
+                          {48, 16, 3, 1, 1},   {54, 9, 3, 2, 1},   {64, 8, 4, 2, 1},   {72, 12, 3, 2, 1},
+                          {96, 8, 6, 2, 1},    {108, 9, 6, 2, 1},  {128, 8, 8, 2, 1},  {144, 9, 8, 2, 1},
+                          {162, 9, 9, 2, 1},   {192, 12, 8, 2, 1}, {216, 12, 9, 2, 1}, {256, 16, 8, 2, 1},
+                          {288, 16, 9, 2, 1},  {324, 12, 9, 3, 1}, {384, 16, 12, 2, 1}, {432, 12, 12, 3, 1},
+                          {512, 16, 16, 2, 1}, {1024, 8, 8, 8, 2}};
+    for (const auto& e : tab)
+      if (e[0] == L) {
+        for (int i = 1; i < 5; ++i)
+          if (e[i] > 1) p.r[p.ns++] = e[i];
+        return p;
+      }
+    return p;  // no plan: ns = 0
+  }
   if (pv == 3) {
     const int tab[][4] = {{12, 4, 3, 1},  {16, 4, 4, 1},   {18, 6, 3, 1},   {24, 6, 4, 1},  {27, 9, 3, 1},
                           {32, 8, 4, 1},  {36, 6, 6, 1},   {48, 8, 6, 1},   {54, 9, 6, 1},  {64, 8, 8, 1},
