@@ -404,15 +404,15 @@ __device__ __forceinline__ const double* ener_tp(const ElxGen&, const DevConst& 
 
 // Row blocks of the final strain: x C2R, then elener with the voxels in row order (the last
 // inverse stage stores every voxel at its own place, after a barrier, so that global memory is
-// read and written in rows; order parameters and P by cp.async during the transform).  mode 0
-// (KKS): elg += el_grad; 1 (Landau): elg = el_grad.  Grid-stride over row blocks: at most PSTRIDE
+// read and written in rows; order parameters and P by cp.async during the transform); the
+// driving force as EnerOut says.  Grid-stride over row blocks: at most PSTRIDE
 // blocks, each one partial of the energy sum.
 template <typename R, int N, typename COEF>
 __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<COEF>()>::BLOCKS))
     k_el_ener(const cplx<R>* __restrict__ sp, int64_t nk, const R* __restrict__ phi, const R* __restrict__ pphi,
               int64_t n3, int64_t nrows, const cplx<R>* __restrict__ tw, const DevConst* __restrict__ Kp,
-              const __grid_constant__ COEF E, R* __restrict__ el_en, R* __restrict__ elg, int mode, int eta2,
-              double* partials, int* err) {
+              const __grid_constant__ COEF E, R* __restrict__ el_en, R* __restrict__ elg,
+              const __grid_constant__ EnerOut<R> out, int eta2, double* partials, int* err) {
   using C = cplx<R>;
   using G = Geo<R, N, is_gen<COEF>()>;
   constexpr int NR = G::NR, NS = fz::rplan(N, PV).ns, NT = G::NT, VS = NR * G::PS;
@@ -470,17 +470,28 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
       ener_stress(E, K, gam, pv, VS, o, err);
       double en = (1.0 - o.psum) * o.mat;
       each_variant(E.nvar, [&](int v) {
-        if (!ener_use(E, K, v)) return;
-        const double elp = ener_ppt(E, K, v, o);
-        en += elp * (double)pv[v * VS];
-        const double* t = ener_tp(E, K, v);
-        const double g = o.sig[0] * t[0] + o.sig[1] * t[1] + o.sig[2] * t[2] +
-                         2.0 * (o.sig[3] * t[3] + o.sig[4] * t[4] + o.sig[5] * t[5]);
         const double f = (double)fv[v * VS];
-        const double pr = eta2 ? 2.0 * f : 30.0 * f * f * (f * f - 2.0 * f + 1.0);
-        const double eg = pr * (o.mat - elp) - g * pr;
-        if (mode == 0) elg[v * n3 + id] += (R)eg;
-        else elg[v * n3 + id] = (R)eg;
+        double eg = 0;
+        if (ener_use(E, K, v)) {
+          const double elp = ener_ppt(E, K, v, o);
+          en += elp * (double)pv[v * VS];
+          const double* t = ener_tp(E, K, v);
+          const double g = o.sig[0] * t[0] + o.sig[1] * t[1] + o.sig[2] * t[2] +
+                           2.0 * (o.sig[3] * t[3] + o.sig[4] * t[4] + o.sig[5] * t[5]);
+          const double pr = eta2 ? 2.0 * f : 30.0 * f * f * (f * f - 2.0 * f + 1.0);
+          eg = pr * (o.mat - elp) - g * pr;
+        } else if (out.mode != 2) {
+          return;
+        }
+        R* d = elg + v * n3 + id;
+        if (out.mode == 2) {
+          const double nz = out.noise ? out.dt * (double)out.noise[v * n3 + id] : 0.0;
+          *d = (R)(f - out.dtl * ((double)*d + eg) + nz);
+        } else if (out.mode == 0) {
+          *d += (R)eg;
+        } else {
+          *d = (R)eg;
+        }
       });
       el_en[id] = (R)en;
       esum += en;
@@ -500,8 +511,8 @@ void launch_rows(const ElRowsArgs<R>& a, const COEF& E, double cfac) {
                                                                  E, (W)cfac, a.err);
 }
 template <typename R, int N, typename COEF>
-void launch_ener(const ElRowsArgs<R>& a, const COEF& E, const R* phi, const DevConst* K, R* el_en, R* elg, int mode,
-                 int eta2, double* partials) {
+void launch_ener(const ElRowsArgs<R>& a, const COEF& E, const R* phi, const DevConst* K, R* el_en, R* elg,
+                 const EnerOut<R>& out, int eta2, double* partials) {
   using G = Geo<R, N, is_gen<COEF>()>;
   auto fn = k_el_ener<R, N, COEF>;
   const size_t sm = (G::line_bytes + 15) / 16 * 16 + sizeof(R) * (size_t)(2 * E.nvar) * G::NR * G::PS;
@@ -509,7 +520,7 @@ void launch_ener(const ElRowsArgs<R>& a, const COEF& E, const R* phi, const DevC
     throw CudaError("elastic energy rows exceed shared memory", MEU_ERR_UNSUPPORTED);
   const unsigned blocks = (unsigned)std::min<int64_t>((a.nrows + G::NR - 1) / G::NR, PSTRIDE);
   fn<<<blocks, G::NT, sm, a.st>>>(a.sp, a.nk, phi, a.pphi, a.n3, a.nrows, (const cplx<R>*)a.tw, K, E, el_en, elg,
-                                         mode, eta2, partials, a.err);
+                                         out, eta2, partials, a.err);
 }
 
 }  // namespace elr

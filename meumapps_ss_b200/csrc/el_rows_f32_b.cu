@@ -20,12 +20,12 @@ bool el_rows_b<float>(const ElRowsArgs<float>& a, const ElRowsCoef<float>& c, do
 }
 template <>
 bool el_ener_b<float>(const ElRowsArgs<float>& a, const ElRowsCoef<float>& c, const float* phi, const DevConst* K, float* el_en,
-                       float* elg, int mode, int eta2, double* partials) {
+                       float* elg, const EnerOut<float>& out, int eta2, double* partials) {
   switch (a.nx) {
 #define MEU_CASE(N)                                                                                    \
   case N:                                                                                              \
-    if (c.prop) elr::launch_ener<float, N, ElenProp>(a, *c.en, phi, K, el_en, elg, mode, eta2, partials); \
-    else elr::launch_ener<float, N, ElxGen>(a, *c.gen, phi, K, el_en, elg, mode, eta2, partials);      \
+    if (c.prop) elr::launch_ener<float, N, ElenProp>(a, *c.en, phi, K, el_en, elg, out, eta2, partials); \
+    else elr::launch_ener<float, N, ElxGen>(a, *c.gen, phi, K, el_en, elg, out, eta2, partials);      \
     return true;
     MEU_ROWS_B(MEU_CASE)
 #undef MEU_CASE

@@ -20,12 +20,12 @@ bool el_rows_a<double>(const ElRowsArgs<double>& a, const ElRowsCoef<double>& c,
 }
 template <>
 bool el_ener_a<double>(const ElRowsArgs<double>& a, const ElRowsCoef<double>& c, const double* phi, const DevConst* K, double* el_en,
-                       double* elg, int mode, int eta2, double* partials) {
+                       double* elg, const EnerOut<double>& out, int eta2, double* partials) {
   switch (a.nx) {
 #define MEU_CASE(N)                                                                                    \
   case N:                                                                                              \
-    if (c.prop) elr::launch_ener<double, N, ElenProp>(a, *c.en, phi, K, el_en, elg, mode, eta2, partials); \
-    else elr::launch_ener<double, N, ElxGen>(a, *c.gen, phi, K, el_en, elg, mode, eta2, partials);      \
+    if (c.prop) elr::launch_ener<double, N, ElenProp>(a, *c.en, phi, K, el_en, elg, out, eta2, partials); \
+    else elr::launch_ener<double, N, ElxGen>(a, *c.gen, phi, K, el_en, elg, out, eta2, partials);      \
     return true;
     MEU_ROWS_A(MEU_CASE)
 #undef MEU_CASE

@@ -310,13 +310,26 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
   // the row kernels: their lengths, proportional moduli or general ones with decoupled normal
   // and shear parts; anything else keeps the real strain and el_x
   el_fused_rows = el_state && el_rows_ok(p.nx) && (hK.prop_moduli || el_ortho_gen);
+  if (p.model == MEU_MODEL_KKS) {
+    kks_axis = axis_ok(p.nx) && axis_ok(p.ny) && axis_ok(p.nz);
+    // off-diagonal gradient coefficients below the rounding of the diagonal's (a rotated
+    // isotropic tensor) do not need the 3-D route
+    kks_lap = V > 1 ? 1 : 0;
+    for (int v = 0; v < V && kks_lap; ++v) {
+      const double* g = p.grad_coeff[v];
+      const double big = std::max(std::fabs(g[0]), std::max(std::fabs(g[4]), std::fabs(g[8])));
+      if (std::fabs(g[3] + g[1]) + std::fabs(g[7] + g[5]) + std::fabs(g[2] + g[6]) > 1e-15 * big) kks_lap = 2;
+    }
+  }
+  if (el_fused_rows || kks_axis) {
+    tw_nx = dalloc<C>(p.nx);
+    std::vector<C> tw(p.nx);
+    fft_twiddles(p.nx, sizeof(R) == 8, tw.data());
+    MEU_CUDA(cudaMemcpy(tw_nx, tw.data(), sizeof(C) * p.nx, cudaMemcpyHostToDevice));
+  }
   if (el_state) {
     if (el_fused_rows) {
       es = dalloc<C>(6 * nk);
-      tw_nx = dalloc<C>(p.nx);
-      std::vector<C> tw(p.nx);
-      fft_twiddles(p.nx, sizeof(R) == 8, tw.data());
-      MEU_CUDA(cudaMemcpy(tw_nx, tw.data(), sizeof(C) * p.nx, cudaMemcpyHostToDevice));
       for (int i = 0; i < 36; ++i) {
         el_gen.c0[i] = hK.c0m[i];
         for (int n = 0; n < p.numph; ++n) el_gen.s[n][i] = p.sela[n][i];
@@ -759,6 +772,7 @@ void Engine<R>::set_fields(const double* cons, const double* phi_in, const doubl
 template <typename R>
 void Engine<R>::add_noise(const double* incr) {
   if (!noise) return;
+  noise_live = true;
   const int64_t chunk = std::max<int64_t>(stage_elems / V, 1);
   for (int64_t v0 = 0; v0 < n3; v0 += chunk) {
     const int64_t nv = std::min(chunk, n3 - v0);
@@ -771,6 +785,7 @@ void Engine<R>::add_noise(const double* incr) {
 // phi_noise += one step's increments already in device memory (Fortran layout)
 template <typename R>
 void Engine<R>::upload_noise(const double* dev_incr) {
+  noise_live = true;
   KLAUNCH("aos_to_soa", (double)n3 * V * (8 + 2 * sizeof(R)),
           k_aos_to_soa<R><<<grid_for(n3 * V, 256), 256, 0, st>>>(dev_incr, noise, V, 0, n3, n3, 1, nullptr));
 }
@@ -865,7 +880,7 @@ void Engine<R>::get_fields(double* cons, double* phi_out, double* el_out, double
 // ---------------------------------------------------------------- elasticity
 // eldis (ModElastic.f:11-489) + elener (:493-691).  P_phi in pphi.
 template <typename R>
-void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only) {
+void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool zeroth_only) {
   const bool first = zeroth_only || step == P.elastep0 || !el_ready;
   // the reference computes the zeroth order only at step == elastep0; a run that
   // enters later without an uploaded state starts from u = 0 like the reference.
@@ -968,27 +983,57 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only)
   if (el_fused_rows) {
     KLAUNCH("elener", 6.0 * nk * sizeof(C) + (double)(2 * V + 1 + V) * n3 * sizeof(R), {
       const ElRowsArgs<R> ra = rows_args();
-      if (!el_ener_a<R>(ra, rows_coef(), ph_for_ppr, dK, el_en, elg, mode, eta2, partials) &&
-          !el_ener_b<R>(ra, rows_coef(), ph_for_ppr, dK, el_en, elg, mode, eta2, partials))
+      if (!el_ener_a<R>(ra, rows_coef(), ph_for_ppr, dK, el_en, elg, eo, eta2, partials) &&
+          !el_ener_b<R>(ra, rows_coef(), ph_for_ppr, dK, el_en, elg, eo, eta2, partials))
         throw CudaError("internal: elastic energy rows for an unsupported length", MEU_ERR_UNSUPPORTED);
     });
   } else if (hK.prop_moduli) {
     KLAUNCH("elener", (double)(2 * V + 6 + 1 + V) * n3 * sizeof(R),
             fn_elener<<<g_elener, PF_TILE, sm_elener, st>>>(en_prop, (int64_t)n3, ph_for_ppr, pphi, strain, el_en, elg,
-                                                            mode, eta2, partials, d_err));
+                                                            eo.mode, eta2, partials, d_err));
   } else
     KLAUNCH("elener", (double)(2 * V + 6 + 1 + V) * n3 * sizeof(R),
             (el_ortho_gen ? k_elener<R, true> : k_elener<R>)<<<g_elener, RED_THREADS, 0, st>>>(
-                dK, ph_for_ppr, pphi, strain, el_en, elg, mode, eta2, partials, d_err));
+                dK, ph_for_ppr, pphi, strain, el_en, elg, eo.mode, eta2, partials, d_err));
 }
 
 // ------------------------------------------------------------------- KKS step
 template <typename R>
 void Engine<R>::kks_step(meu_diag* d) {
   MEU_CUDA(cudaMemsetAsync(partials, 0, sizeof(double) * Q_TOTAL * PSTRIDE, st));
-  if (!(step <= P.noise_step)) MEU_CUDA(cudaMemsetAsync(noise, 0, sizeof(R) * V * n3, st));
+  if (!(step <= P.noise_step) && noise_live) {
+    MEU_CUDA(cudaMemsetAsync(noise, 0, sizeof(R) * V * n3, st));
+    noise_live = false;
+  }
   // spectral gradients (:575-615)
-  {
+  if (kks_axis) {
+    AxisArgs<R> A{};
+    A.f = phi;
+    A.fs = n3;
+    A.os = A.ls = 4 * n3;
+    for (int v = 0; v < V; ++v) A.s[v] = 1.0;
+    for (int d = 0; d < 3; ++d) {
+      A.out = field(wr, d);
+      if (kks_lap == 1) {
+        A.lap = field(wr, 3);
+        A.lap_add = d > 0;
+        for (int v = 0; v < V; ++v) A.g[v] = P.grad_coeff[v][4 * d];
+      }
+      KLAUNCH("kks_grad", (double)V * (kks_lap == 1 ? 3 + (d > 0) : 2) * n3 * sizeof(R),
+              axis_launch<R>(d, A, V, *fft, tw_nx, st));
+    }
+    if (kks_lap == 2) {
+      std::vector<const R*> in;
+      std::vector<R*> out;
+      for (int v = 0; v < V; ++v) {
+        in.push_back(field(phi, v));
+        out.push_back(field(wr, 4 * v + 3));
+      }
+      fwd_list(in, 0);
+      KLAUNCH("kks_lap", 2.0 * V * nk * sizeof(C), k_kks_lap<R><<<gridk(), 256, 0, st>>>(dK, spec(0), V));
+      inv_list(0, out);
+    }
+  } else {
     std::vector<const R*> in;
     for (int v = 0; v < V; ++v) in.push_back(field(phi, v));
     fwd_list(in, 0);
@@ -1007,24 +1052,75 @@ void Engine<R>::kks_step(meu_diag* d) {
     KLAUNCH("kks_point", (double)(7 * V + 4 * E) * n3 * sizeof(R),
             kp<<<RED_BLOCKS, RED_THREADS, 0, st>>>(dK, phi, c, wr, pphi, fd, fc, partials, d_err));
   }
-  // elasticity (:851-880)
+  // elasticity (:851-880); on the row path elener writes the TDGL right-hand side into fd
   last_iters = 0;
+  bool rhs_done = false;
   if (step >= P.elastep0 && P.elastic != MEU_ELAST_NONE) {
-    elastic(phi, fd, 0, false);
+    rhs_done = el_fused_rows;
+    elastic(phi, fd, EnerOut<R>{rhs_done ? 2 : 0, P.dt * P.b_mob, P.dt, noise_live ? noise : nullptr}, false);
   } else {
     MEU_CUDA(cudaMemsetAsync(el_en, 0, sizeof(R) * n3, st));
   }
-  // diffusion (:910-949)
-  for (int e = 0; e < E; ++e) {
-    fwd({field(c, e), field(fc, 3 * e), field(fc, 3 * e + 1), field(fc, 3 * e + 2)}, 0);
-    KLAUNCH("kks_ch", 5.0 * nk * sizeof(C), k_kks_ch<R><<<gridk(), 256, 0, st>>>(dK, spec(0), spec(1), spec(2), spec(3), P.dt * P.cmobs[e]));
-    inv_list(0, {field(c, e)});
-  }
-  // TDGL (:955-1001)
-  KLAUNCH("tdgl_pre", 4.0 * V * n3 * sizeof(R), k_tdgl_pre<R><<<grid_for((int64_t)V * n3, 256), 256, 0, st>>>(phi, fd, noise, wr, (int64_t)V * n3, P.dt * P.b_mob, P.dt));
-  {
+  if (kks_axis) {
+    // w_c = C + dt M div F (:910-949) in wr[0..E), w_phi = phi - dt L f + dt noise (:955-1001) in
+    // fd or wr[E..E+V); then one forward, division and inverse of all of them
+    AxisArgs<R> A{};
+    A.fs = 3 * n3;
+    A.os = A.as = A.bs = n3;
+    A.out = wr;
+    for (int d = 0; d < 3; ++d) {
+      A.f = field(fc, d);
+      if (d == 1) A.acc = wr;
+      if (d == 2) A.base = c;
+      for (int e = 0; e < E; ++e) A.s[e] = d == 2 ? P.dt * P.cmobs[e] : 1.0;
+      KLAUNCH("kks_div", (double)E * (2 + d) * n3 * sizeof(R), axis_launch<R>(d, A, E, *fft, tw_nx, st));
+    }
+    R* wp = rhs_done ? fd : field(wr, E);
+    if (!rhs_done)
+      KLAUNCH("tdgl_pre", 4.0 * V * n3 * sizeof(R), k_tdgl_pre<R><<<grid_for((int64_t)V * n3, 256), 256, 0, st>>>(phi, fd, noise, wp, (int64_t)V * n3, P.dt * P.b_mob, P.dt));
+    ZDivArgs<R> Z{};
+    Z.sp = spec(0);
+    Z.stride = nk;
+    Z.inner = P.ny * hK.nxh;
+    Z.nxh = hK.nxh;
+    Z.nx = P.nx;
+    Z.ny = P.ny;
+    Z.scale = 1.0 / ((double)P.nx * P.ny * P.nz);
+    Z.wx = 6.283185307179586476925286766559 / (double)P.nx;
+    Z.wy = 6.283185307179586476925286766559 / (double)P.ny;
+    PtrList<const R> in{};
+    PtrList<R> out{};
+    for (int e = 0; e < E; ++e) {
+      in.p[e] = field(wr, e);
+      out.p[e] = field(c, e);
+      Z.s[e] = P.dt * P.cmobs[e];
+      Z.g[e][0] = Z.g[e][4] = Z.g[e][8] = 1.0;
+    }
+    for (int v = 0; v < V; ++v) {
+      in.p[E + v] = wp + (int64_t)v * n3;
+      out.p[E + v] = field(phi, v);
+      Z.s[E + v] = P.dt * P.b_mob;
+      for (int i = 0; i < 9; ++i) Z.g[E + v][i] = P.grad_coeff[v][i];
+    }
+    const PtrList<C> S = specs(0, E + V);
+    fft->forward_x<R>(in, S, E + V, st);
+    fft->pass_y<R>(S, E + V, true, st);
+    KLAUNCH("kks_zdiv", 2.0 * (E + V) * nk * sizeof(C), z_div_launch<R>(Z, E + V, *fft, st));
+    fft->pass_y<R>(S, E + V, false, st);
+    fft->inverse_x<R>(S, out, E + V, st);
+  } else {
+    // diffusion (:910-949)
+    for (int e = 0; e < E; ++e) {
+      fwd({field(c, e), field(fc, 3 * e), field(fc, 3 * e + 1), field(fc, 3 * e + 2)}, 0);
+      KLAUNCH("kks_ch", 5.0 * nk * sizeof(C), k_kks_ch<R><<<gridk(), 256, 0, st>>>(dK, spec(0), spec(1), spec(2), spec(3), P.dt * P.cmobs[e]));
+      inv_list(0, {field(c, e)});
+    }
+    // TDGL (:955-1001)
+    R* wp = rhs_done ? fd : wr;
+    if (!rhs_done)
+      KLAUNCH("tdgl_pre", 4.0 * V * n3 * sizeof(R), k_tdgl_pre<R><<<grid_for((int64_t)V * n3, 256), 256, 0, st>>>(phi, fd, noise, wp, (int64_t)V * n3, P.dt * P.b_mob, P.dt));
     std::vector<const R*> in;
-    for (int v = 0; v < V; ++v) in.push_back(field(wr, v));
+    for (int v = 0; v < V; ++v) in.push_back(field(wp, v));
     fwd_list(in, 0);
     KLAUNCH("tdgl", 2.0 * V * nk * sizeof(C), k_tdgl<R><<<gridk(), 256, 0, st>>>(dK, specs(0, V), V, P.dt * P.b_mob));
     std::vector<R*> out;
@@ -1209,7 +1305,7 @@ void Engine<R>::landau_step(meu_diag* d) {
   last_iters = 0;
   if (het) {
     // P_phi = theta (already in pphi), elener gives el_grad into phel
-    elastic(phi, phel, 1, false);
+    elastic(phi, phel, EnerOut<R>{1, 0.0, 0.0, nullptr}, false);
   } else if (!homog) {
     MEU_CUDA(cudaMemsetAsync(el_en, 0, sizeof(R) * n3, st));
   }

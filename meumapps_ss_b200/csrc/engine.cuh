@@ -66,6 +66,44 @@ int el_z_blocks(int nz, int inner);
 // sp: six contiguous spectra; part: [6][el_z_blocks] partial sums of the convergence test
 template <typename R>
 void el_z_launch(const FFT3& f, cplx<R>* sp, cplx<R>* uk, const ElzCoef& E, double* part, cudaStream_t st);
+// derivatives along one axis (deriv.cuh): field v of the launch at f + v * fs;
+// out = base + s (acc + D f), lap (+)= g D2 f (NULL: not formed)
+template <typename R>
+struct AxisArgs {
+  const R* f;
+  R* out;
+  const R *acc, *base;
+  R* lap;
+  int64_t fs, os, as, bs, ls;
+  double s[MEU_MAX_VAR], g[MEU_MAX_VAR];
+  int lap_add;
+};
+inline bool axis_ok(int n) {
+  for (int l : {16, 24, 32, 36, 48, 54, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 512})
+    if (n == l) return true;
+  return false;
+}
+template <typename R>
+void axis_launch(int axis, const AxisArgs<R>& A, int nf, const FFT3& f, const void* tw_nx, cudaStream_t st);
+// z FFT, division by 1 + s k.kappa.k (times scale), z inverse FFT of nf spectra
+template <typename R>
+struct ZDivArgs {
+  cplx<R>* sp;
+  int64_t stride;
+  int inner, nxh, nx, ny;
+  double scale, wx, wy;
+  double s[MEU_MAX_VAR + MEU_MAX_EL], g[MEU_MAX_VAR + MEU_MAX_EL][9];
+};
+template <typename R>
+void z_div_launch(const ZDivArgs<R>& A, int nf, const FFT3& f, cudaStream_t st);
+// what elener does with the driving force eg: 0 elg += eg; 1 elg = eg; 2 the right-hand side of
+// the TDGL update, elg = phi - dtl (elg + eg) + dt noise (Multi_MEUMAPPS.f:957-987)
+template <typename R>
+struct EnerOut {
+  int mode;
+  double dtl, dt;
+  const R* noise;  // NULL: zero
+};
 // x-direction work of one elastic iteration in one pass, and elener on the same row spectra
 // (el_rows.cuh): sp the six row spectra, nk apart; tw: exp(-2 pi i n / nx), n < nx
 template <typename R>
@@ -93,10 +131,10 @@ template <typename R>
 bool el_rows_b(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, double cfac, bool fp64);
 template <typename R>
 bool el_ener_a(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, const R* phi, const DevConst* K, R* el_en, R* elg,
-               int mode, int eta2, double* partials);
+               const EnerOut<R>& out, int eta2, double* partials);
 template <typename R>
 bool el_ener_b(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, const R* phi, const DevConst* K, R* el_en, R* elg,
-               int mode, int eta2, double* partials);
+               const EnerOut<R>& out, int eta2, double* partials);
 inline bool el_rows_ok(int nx) {
   for (int n : {16, 24, 32, 36, 48, 54, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 512, 1024})
     if (nx == n) return true;
@@ -324,7 +362,7 @@ class Engine : public EngineBase {
   }
   void check_err();
   void finalize(int q0, int nq, double* out = nullptr, const int* nbs = nullptr);
-  void elastic(const R* ph_for_ppr, R* elg, int mode, bool zeroth_only);
+  void elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& out, bool zeroth_only);
   void kks_step(meu_diag* d);
   void landau_step(meu_diag* d);
   void landau_step_fused();
@@ -359,6 +397,12 @@ class Engine : public EngineBase {
   // iterations run the x direction as one kernel on the row spectra es (six, nk apart), which
   // replace the real strain and polarisation fields
   bool el_fused_rows = false;
+  // KKS: gradients, Laplacians and flux divergence by one-axis transforms (every side has them);
+  // kappa-Laplacian: 0 not needed (one variant), 1 per axis (diagonal gradient tensors), 2 by
+  // the 3-D transform
+  bool kks_axis = false;
+  int kks_lap = 0;
+  bool noise_live = false;            // phi_noise may be nonzero
   bool el_state = false;              // heterogeneous elasticity keeps a state between steps
   C* es = nullptr;
   C* tw_nx = nullptr;                 // exp(-2 pi i n / nx), n < nx

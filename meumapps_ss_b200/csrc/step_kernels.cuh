@@ -40,6 +40,24 @@ __global__ void __launch_bounds__(256) k_kks_grad(const DevConst* __restrict__ K
   }
 }
 
+// kappa-Laplacian alone, in place (gradient tensors with off-diagonal entries; the gradients
+// then come from one-axis transforms)
+template <typename R>
+__global__ void __launch_bounds__(256) k_kks_lap(const DevConst* __restrict__ Kp, cplx<R>* __restrict__ sp, int V) {
+  const DevConst& K = *Kp;
+  for (int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < K.nk; id += (int64_t)gridDim.x * blockDim.x) {
+    int kx, ky, kz;
+    kdecode(K, id, kx, ky, kz);
+    double a[3], b[3];
+    kvec(K, kx, ky, kz, a, b);
+    for (int v = 0; v < V; ++v) {
+      const cplx<R> val = sp[v * K.nk + id];
+      const double m = -kkappak(K.p.grad_coeff[v], a, b);
+      sp[v * K.nk + id] = mk((R)((double)val.x * m), (R)((double)val.y * m));
+    }
+  }
+}
+
 // ------------------------------------------------- KKS: local driving force
 // Multi_MEUMAPPS.f:634-845 per voxel.  g4 = [gx_v, gy_v, gz_v, kds_v] per v.
 // Fields in R; the local solve and the energies in FP64.  NPH, NEL > 0: the phase and
