@@ -4,14 +4,14 @@
 namespace meu {
 
 template <>
-bool el_rows_a<double>(const ElRowsArgs<double>& a, const ElRowsCoef<double>& c, double cfac, bool fp64) {
+bool el_rows_a<double>(const ElRowsArgs<double>& a, const ElRowsCoef<double>& c, bool fp64) {
   (void)fp64;  // FP64 fields have one precision
   switch (a.nx) {
 #define MEU_CASE(N)                                                                          \
   case N:                                                                                    \
-    if (!c.prop) elr::launch_rows<double, N, double, ElxGen>(a, *c.gen, cfac);                \
-    else if (sizeof(double) == 4 && fp64) elr::launch_rows<double, N, double, ElxProp>(a, *c.p64, cfac); \
-    else elr::launch_rows<double, N, double, ElxCoef<double>>(a, *c.pr, cfac);                     \
+    if (!c.prop) elr::launch_rows<double, N, double, ElxGen>(a, *c.gen);                \
+    else if (sizeof(double) == 4 && fp64) elr::launch_rows<double, N, double, ElxProp>(a, *c.p64); \
+    else elr::launch_rows<double, N, double, ElxCoef<double>>(a, *c.pr);                     \
     return true;
     MEU_ROWS_A(MEU_CASE)
 #undef MEU_CASE

@@ -91,12 +91,64 @@ __global__ void __launch_bounds__(256) k_el_qcheck(const DevConst* __restrict__ 
     set_err(err, invert3(Q, MEU_ERR_Q_SINGULAR));
   }
 }
-// the six convergence sums from k_el_z's block partials, in a fixed order
-__global__ void __launch_bounds__(1024) k_el_zsum(const double* __restrict__ part, int nblk, double* out) {
+// One iteration's outcome (ModElastic.f:435-481): convergence, backtracking with the damping
+// halved, the ramp of the damping back to 1.  sums: the six convergence sums over n3.
+__device__ void el_control(const ElCtlArgs& A, const double* sums) {
+  ElCtl& c = *A.ctl;
+  if (A.first) {
+    c.cfac = 1.0;
+    c.newfac = 0.5;
+    c.niter = c.total = c.converged = c.status = 0;
+    for (int q = 0; q < 6; ++q) c.err_old[q] = 0.0;
+  }
+  c.done = 0;
+  c.niter += 1;
+  c.total += 1;
+  double e[6];
+  for (int q = 0; q < 6; ++q) e[q] = sums[q] * A.n3;
+  if (e[0] / e[1] < A.tol && e[2] / e[3] < A.tol && e[4] / e[5] < A.tol) c.converged = 1;
+  if (c.niter > 1 && !c.converged) {
+    const double* o = c.err_old;
+    if (e[0] / e[1] > o[0] / o[1] || e[2] / e[3] > o[2] / o[3] || e[4] / e[5] > o[4] / o[5]) {
+      c.cfac = c.cfac * c.newfac;
+      c.newfac = c.newfac * 0.5;
+      if (c.newfac < 1e-7) c.status = MEU_ERR_NOT_CONVERGED;
+      c.niter = 0;
+      c.converged = 0;
+      return;
+    }
+  }
+  for (int q = 0; q < 6; ++q) c.err_old[q] = e[q];
+  if (c.niter == A.max_iter) c.converged = 1;
+  if (!c.converged || c.niter < A.min_iter) return;
+  if (c.cfac < 1.0 - 1e-6) {
+    c.cfac = c.cfac + 0.1;
+    if (c.cfac > 1.0) c.cfac = 1.0;
+    c.niter = 0;
+    c.converged = 0;
+    return;
+  }
+  c.done = 1;
+}
+// the six convergence sums from k_el_z's block partials, in a fixed order (block q sums q);
+// the last block to finish runs the control
+__global__ void __launch_bounds__(1024) k_el_zsum(const double* __restrict__ part, int nblk, double* out, unsigned* ticket,
+                                                  const __grid_constant__ ElCtlArgs A) {
   const double* p = part + (int64_t)blockIdx.x * nblk;
   double acc = 0;
   for (int i = threadIdx.x; i < nblk; i += blockDim.x) acc += p[i];
   block_reduce_store(acc, 0, out + blockIdx.x);
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(ticket, 1u) != gridDim.x - 1) return;
+  *ticket = 0;
+  __threadfence();
+  double s[6];
+  for (int q = 0; q < 6; ++q) s[q] = __ldcg(out + q);
+  el_control(A, s);
+}
+__global__ void k_el_control(const double* sums, const __grid_constant__ ElCtlArgs A) {
+  if (threadIdx.x == 0) el_control(A, sums);
 }
 
 // the fluctuation spectrum has no k = 0 mode
@@ -361,7 +413,12 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
   hist = dalloc<double>((int64_t)HIST_MAX * Q_STEP_COUNT);
   cmean_acc = dalloc<double>(MEU_MAX_EL);
   d_ops = dalloc<int>(Q_TOTAL);
-  d_err = dalloc<int>(1);
+  d_ctl = dalloc<ElCtl>(1);
+  d_err = &d_ctl->err;
+  el_ticket = dalloc<unsigned>(1);
+  MEU_CUDA(cudaMemset(d_ctl, 0, sizeof(ElCtl)));
+  MEU_CUDA(cudaMemset(el_ticket, 0, sizeof(unsigned)));
+  MEU_CUDA(cudaHostAlloc((void**)&h_ctl, sizeof(ElCtl), cudaHostAllocDefault));
   dK = dalloc<DevConst>(1);
   MEU_CUDA(cudaHostAlloc((void**)&h_results, sizeof(double) * Q_TOTAL, cudaHostAllocDefault));
   MEU_CUDA(cudaHostAlloc((void**)&h_err, sizeof(int), cudaHostAllocDefault));
@@ -636,6 +693,7 @@ Engine<R>::~Engine() {
   for (void* q : allocs) cudaFree(q);
   if (h_results) cudaFreeHost(h_results);
   if (h_err) cudaFreeHost(h_err);
+  if (h_ctl) cudaFreeHost(h_ctl);
   for (int b = 0; b < 2; ++b) {
     if (noise_host[b]) cudaFreeHost(noise_host[b]);
     if (noise_ev[b]) cudaEventDestroy(noise_ev[b]);
@@ -648,12 +706,13 @@ template <typename R>
 void Engine<R>::check_err() {
   MEU_CUDA(cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   MEU_CUDA(cudaStreamSynchronize(st));
-  if (*h_err) {
-    int code = *h_err;
-    MEU_CUDA(cudaMemset(d_err, 0, sizeof(int)));
-    if (code == MEU_ERR_TIMEOUT) throw CudaError("a bounded device-side wait ran out in the step", code);
-    throw CudaError("singular matrix in the step (reference err_flag " + std::to_string(code) + ")", code);
-  }
+  if (*h_err) raise_err(*h_err);
+}
+template <typename R>
+void Engine<R>::raise_err(int code) {
+  MEU_CUDA(cudaMemset(d_err, 0, sizeof(int)));
+  if (code == MEU_ERR_TIMEOUT) throw CudaError("a bounded device-side wait ran out in the step", code);
+  throw CudaError("singular matrix in the step (reference err_flag " + std::to_string(code) + ")", code);
 }
 
 template <typename R>
@@ -903,79 +962,65 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
   el_ready = true;
   int total = 0;
   if (!zeroth_only) {
-    double newfac = 0.5, cfac = 1.0, err_old[6] = {0, 0, 0, 0, 0, 0};
-    int niter = 0;
-    bool converged = false;
+    // The control runs on the device.  An iteration before the el_min_iter'th cannot end the
+    // loop, so on the row path (whose damping the kernels read from the device) those are queued
+    // together: one wait of the host per step instead of one per iteration where el_min_iter
+    // suffice.
+    double cfac = 1.0;
     for (;;) {
-      niter += 1;
-      total += 1;
-      if (total > 100000) throw CudaError("elastic iteration runaway", MEU_ERR_NOT_CONVERGED);
-      // ---- polarisation and its x transform
-      if (el_fused_rows) {
-        // the first iteration's polarisation in FP64 whatever the fields' precision
-        KLAUNCH("el_rows", 6.0 * 2 * nk * sizeof(C) + (double)V * n3 * sizeof(R), {
-          const ElRowsArgs<R> ra = rows_args();
-          if (!el_rows_a<R>(ra, rows_coef(), cfac, total == 1) && !el_rows_b<R>(ra, rows_coef(), cfac, total == 1))
-            throw CudaError("internal: fused elastic rows for an unsupported length", MEU_ERR_UNSUPPORTED);
-        });
-      } else {
-        if (hK.prop_moduli) {
-          KLAUNCH("el_x", (double)(V + 12) * n3 * sizeof(R),
-                  fn_el_x<<<g_el_x, PF_TILE, sm_el_x, st>>>(el_prop, (int64_t)n3, pphi, strain, xs, cfac, d_err));
-        } else
-          KLAUNCH("el_x", (double)(V + 12) * n3 * sizeof(R),
-                  (el_ortho_gen ? k_el_x<R, true> : k_el_x<R>)<<<gridr(), 256, 0, st>>>(dK, pphi, strain, xs, cfac, d_err));
-        PtrList<const R> in{};
-        for (int m = 0; m < 6; ++m) in.p[m] = field(xs, m);
-        fft->forward_x<R>(in, S6, 6, st);
-      }
-      // ---- y, k-space, y
-      fft->pass_y<R>(S6, 6, true, st);
-      if (elz_blocks) {
-        if (!elz_q_checked) KLAUNCH("el_qcheck", 0.0, k_el_qcheck<<<gridk(), 256, 0, st>>>(dK, d_err));
-        KLAUNCH("el_z", 18.0 * nk * sizeof(C), el_z_launch<R>(*fft, S6.p[0], uk, elz, elz_part, st));
-        KLAUNCH("finalize", 48.0 * elz_blocks, k_el_zsum<<<6, 1024, 0, st>>>(elz_part, elz_blocks, results + Q_ERR0));
-      } else {
-        fft->pass_z<R>(S6, 6, true, st);
-        KLAUNCH("el_k", 18.0 * nk * sizeof(C), k_el_k<R><<<g_el_k, RED_THREADS, 0, st>>>(dK, S6, uk, partials, d_err));
-        fft->pass_z<R>(S6, 6, false, st);
-        finalize(Q_ERR0, 6);
-      }
-      fft->pass_y<R>(S6, 6, false, st);
-      if (!el_fused_rows) {
-        PtrList<R> o{};
-        for (int m = 0; m < 6; ++m) o.p[m] = out[m];
-        fft->inverse_x<R>(S6, o, 6, st);
-      }
-      MEU_CUDA(cudaMemcpyAsync(h_results + Q_ERR0, results + Q_ERR0, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
-      check_err();  // synchronises
-      elz_q_checked = elz_blocks > 0;
-      double err[6];
-      for (int q = 0; q < 6; ++q) err[q] = h_results[Q_ERR0 + q] * (double)n3;
-      const double tol = P.el_tol;
-      if (err[0] / err[1] < tol && err[2] / err[3] < tol && err[4] / err[5] < tol) converged = true;
-      if (niter > 1 && !converged) {
-        if (err[0] / err[1] > err_old[0] / err_old[1] || err[2] / err[3] > err_old[2] / err_old[3] ||
-            err[4] / err[5] > err_old[4] / err_old[5]) {
-          cfac = cfac * newfac;
-          newfac = newfac * 0.5;
-          if (newfac < 1e-7) throw CudaError("newfac is too small ... trouble converging", MEU_ERR_NOT_CONVERGED);
-          niter = 0;
-          converged = false;
-          continue;
+      const int batch = el_fused_rows && total == 0 ? std::max(1, P.el_min_iter) : 1;
+      for (int i = 0; i < batch; ++i) {
+        total += 1;
+        if (total > 100000) throw CudaError("elastic iteration runaway", MEU_ERR_NOT_CONVERGED);
+        // ---- polarisation and its x transform
+        if (el_fused_rows) {
+          // the first iteration's polarisation in FP64 whatever the fields' precision
+          KLAUNCH("el_rows", 6.0 * 2 * nk * sizeof(C) + (double)V * n3 * sizeof(R), {
+            ElRowsArgs<R> ra = rows_args();
+            ra.cfac = total == 1 ? nullptr : &d_ctl->cfac;
+            if (!el_rows_a<R>(ra, rows_coef(), total == 1) && !el_rows_b<R>(ra, rows_coef(), total == 1))
+              throw CudaError("internal: fused elastic rows for an unsupported length", MEU_ERR_UNSUPPORTED);
+          });
+        } else {
+          if (hK.prop_moduli) {
+            KLAUNCH("el_x", (double)(V + 12) * n3 * sizeof(R),
+                    fn_el_x<<<g_el_x, PF_TILE, sm_el_x, st>>>(el_prop, (int64_t)n3, pphi, strain, xs, cfac, d_err));
+          } else
+            KLAUNCH("el_x", (double)(V + 12) * n3 * sizeof(R),
+                    (el_ortho_gen ? k_el_x<R, true> : k_el_x<R>)<<<gridr(), 256, 0, st>>>(dK, pphi, strain, xs, cfac, d_err));
+          PtrList<const R> in{};
+          for (int m = 0; m < 6; ++m) in.p[m] = field(xs, m);
+          fft->forward_x<R>(in, S6, 6, st);
+        }
+        // ---- y, k-space, y
+        const ElCtlArgs ca{d_ctl, P.el_tol, (double)n3, P.el_min_iter, P.el_max_iter, total == 1 ? 1 : 0};
+        fft->pass_y<R>(S6, 6, true, st);
+        if (elz_blocks) {
+          if (!elz_q_checked && i == 0) KLAUNCH("el_qcheck", 0.0, k_el_qcheck<<<gridk(), 256, 0, st>>>(dK, d_err));
+          KLAUNCH("el_z", 18.0 * nk * sizeof(C), el_z_launch<R>(*fft, S6.p[0], uk, elz, elz_part, st));
+          KLAUNCH("finalize", 48.0 * elz_blocks,
+                  k_el_zsum<<<6, 1024, 0, st>>>(elz_part, elz_blocks, results + Q_ERR0, el_ticket, ca));
+        } else {
+          fft->pass_z<R>(S6, 6, true, st);
+          KLAUNCH("el_k", 18.0 * nk * sizeof(C), k_el_k<R><<<g_el_k, RED_THREADS, 0, st>>>(dK, S6, uk, partials, d_err));
+          fft->pass_z<R>(S6, 6, false, st);
+          finalize(Q_ERR0, 6);
+          KLAUNCH("finalize", 48.0, k_el_control<<<1, 32, 0, st>>>(results + Q_ERR0, ca));
+        }
+        fft->pass_y<R>(S6, 6, false, st);
+        if (!el_fused_rows) {
+          PtrList<R> o{};
+          for (int m = 0; m < 6; ++m) o.p[m] = out[m];
+          fft->inverse_x<R>(S6, o, 6, st);
         }
       }
-      memcpy(err_old, err, sizeof(err));
-      if (niter == P.el_max_iter) converged = true;
-      if (!converged || niter < P.el_min_iter) continue;
-      if (cfac < 1.0 - 1e-6) {
-        cfac = cfac + 0.1;
-        if (cfac > 1.0) cfac = 1.0;
-        niter = 0;
-        converged = false;
-        continue;
-      }
-      break;
+      MEU_CUDA(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(ElCtl), cudaMemcpyDeviceToHost, st));
+      MEU_CUDA(cudaStreamSynchronize(st));
+      if (h_ctl->err) raise_err(h_ctl->err);
+      elz_q_checked = elz_blocks > 0;
+      if (h_ctl->status) throw CudaError("newfac is too small ... trouble converging", h_ctl->status);
+      if (h_ctl->done) break;
+      cfac = h_ctl->cfac;
     }
   }
   last_iters = total;

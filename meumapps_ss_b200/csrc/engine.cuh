@@ -60,6 +60,18 @@ struct ElzCoef {
   double q[6][6], qs, scale, wx, wy;
   int nx, ny, nxh, inner, ortho;
 };
+// Control of the fixed point (ModElastic.f:435-481), kept on the device so that iterations which
+// cannot be the last are queued without the host: the damping cfac of the next iteration, and
+// the last one's outcome.  err is the step's error word (d_err points at it).
+struct ElCtl {
+  double cfac, newfac, err_old[6];
+  int niter, total, converged, done, status, err;
+};
+struct ElCtlArgs {
+  ElCtl* ctl;
+  double tol, n3;
+  int min_iter, max_iter, first;  // first: the step's first iteration
+};
 // blocks of the z kernel (each writes six partial sums); 0: no kernel for the length
 template <typename R>
 int el_z_blocks(int nz, int inner);
@@ -113,6 +125,7 @@ struct ElRowsArgs {
   const void* tw;
   int64_t nk, n3, nrows;
   int nx;
+  const double* cfac;  // device; NULL: 1
   int* err;
   cudaStream_t st;
 };
@@ -126,9 +139,9 @@ struct ElRowsCoef {
 };
 // false: no kernel for nx (a: up to 128, b: longer).  fp64: the polarisation in FP64.
 template <typename R>
-bool el_rows_a(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, double cfac, bool fp64);
+bool el_rows_a(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, bool fp64);
 template <typename R>
-bool el_rows_b(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, double cfac, bool fp64);
+bool el_rows_b(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, bool fp64);
 template <typename R>
 bool el_ener_a(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, const R* phi, const DevConst* K, R* el_en, R* elg,
                const EnerOut<R>& out, int eta2, double* partials);
@@ -302,6 +315,8 @@ class Engine : public EngineBase {
   int* d_ops = nullptr;
   int* d_err = nullptr;
   int* h_err = nullptr;
+  ElCtl *d_ctl = nullptr, *h_ctl = nullptr;  // h_ctl pinned
+  unsigned* el_ticket = nullptr;
   double* stage = nullptr;  // AoS staging (double)
   // run_noise: two pinned host buffers of one step's increments (Fortran layout), their
   // device copy, and the events that free a host buffer once its copy has run
@@ -361,6 +376,7 @@ class Engine : public EngineBase {
     return l;
   }
   void check_err();
+  void raise_err(int code);  // clears the device's error word and throws
   void finalize(int q0, int nq, double* out = nullptr, const int* nbs = nullptr);
   void elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& out, bool zeroth_only);
   void kks_step(meu_diag* d);
@@ -408,7 +424,7 @@ class Engine : public EngineBase {
   C* tw_nx = nullptr;                 // exp(-2 pi i n / nx), n < nx
   ElxGen el_gen{};
   ElRowsArgs<R> rows_args() const {
-    return {es, pphi, tw_nx, nk, n3, (int64_t)P.ny * P.nz, P.nx, d_err, st};
+    return {es, pphi, tw_nx, nk, n3, (int64_t)P.ny * P.nz, P.nx, nullptr, d_err, st};
   }
   ElRowsCoef<R> rows_coef() const { return {hK.prop_moduli != 0, &el_prop_r, &el_prop, &en_prop, &el_gen}; }
   PtrList<C> es_list() const {
