@@ -487,7 +487,8 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
         R* d = elg + v * n3 + id;
         if (out.mode == 2) {
           const double nz = out.noise ? out.dt * (double)out.noise[v * n3 + id] : 0.0;
-          *d = (R)(f - out.dtl * ((double)*d + eg) + nz);
+          const R t = *d + (R)eg;  // the force in the fields' precision, as mode 0 leaves it
+          *d = (R)(f - out.dtl * (double)t + nz);
         } else if (out.mode == 0) {
           *d += (R)eg;
         } else {

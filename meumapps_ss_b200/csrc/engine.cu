@@ -361,13 +361,15 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
   el_state = elast && het;
   // the row kernels: their lengths, proportional moduli or general ones with decoupled normal
   // and shear parts; anything else keeps the real strain and el_x
-  el_fused_rows = el_state && el_rows_ok(p.nx) && (hK.prop_moduli || el_ortho_gen);
+  keep_rounding = p.model == MEU_MODEL_KKS && sizeof(R) == 4 && V > 1;
+  fft->mix = !keep_rounding;
+  el_fused_rows = el_state && !keep_rounding && el_rows_ok(p.nx) && (hK.prop_moduli || el_ortho_gen);
   if (p.model == MEU_MODEL_KKS) {
-    kks_axis = axis_ok(p.nx) && axis_ok(p.ny) && axis_ok(p.nz);
+    kks_axis = !keep_rounding && axis_ok(p.nx) && axis_ok(p.ny) && axis_ok(p.nz);
     // off-diagonal gradient coefficients below the rounding of the diagonal's (a rotated
     // isotropic tensor) do not need the 3-D route
-    kks_lap = V > 1 ? 1 : 0;
-    for (int v = 0; v < V && kks_lap; ++v) {
+    kks_lap = V == 1 ? 0 : 1;
+    for (int v = 0; v < V && kks_lap == 1; ++v) {
       const double* g = p.grad_coeff[v];
       const double big = std::max(std::fabs(g[0]), std::max(std::fabs(g[4]), std::fabs(g[8])));
       if (std::fabs(g[3] + g[1]) + std::fabs(g[7] + g[5]) + std::fabs(g[2] + g[6]) > 1e-15 * big) kks_lap = 2;
@@ -513,6 +515,9 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
       for (int i = 0; i < 6; ++i)
         for (int j = 0; j < i; ++j) sym = sym && hK.c0m[i + j * 6] == hK.c0m[j + i * 6];
       elz_blocks = sym ? el_z_blocks<R>(p.nz, p.ny * hK.nxh) : 0;
+      // (its plan and scaling are the separate passes' where nz is 32 or 64 and the cell count a
+      // power of two)
+      if (keep_rounding && !((p.nz == 32 || p.nz == 64) && (n3 & (n3 - 1)) == 0)) elz_blocks = 0;
       if (elz_blocks) {
         elz_part = dalloc<double>(6 * (int64_t)elz_blocks);
         int ex = 0;
@@ -963,13 +968,12 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
   int total = 0;
   if (!zeroth_only) {
     // The control runs on the device.  An iteration before the el_min_iter'th cannot end the
-    // loop, so on the row path (whose damping the kernels read from the device) those are queued
-    // together: one wait of the host per step instead of one per iteration where el_min_iter
-    // suffice.
-    double cfac = 1.0;
+    // loop, so those are queued together: one wait of the host per step instead of one per
+    // iteration where el_min_iter suffice.
     for (;;) {
-      const int batch = el_fused_rows && total == 0 ? std::max(1, P.el_min_iter) : 1;
+      const int batch = total == 0 ? std::max(1, P.el_min_iter) : 1;
       for (int i = 0; i < batch; ++i) {
+        const double* cfac = total == 0 ? nullptr : &d_ctl->cfac;
         total += 1;
         if (total > 100000) throw CudaError("elastic iteration runaway", MEU_ERR_NOT_CONVERGED);
         // ---- polarisation and its x transform
@@ -977,7 +981,7 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
           // the first iteration's polarisation in FP64 whatever the fields' precision
           KLAUNCH("el_rows", 6.0 * 2 * nk * sizeof(C) + (double)V * n3 * sizeof(R), {
             ElRowsArgs<R> ra = rows_args();
-            ra.cfac = total == 1 ? nullptr : &d_ctl->cfac;
+            ra.cfac = cfac;
             if (!el_rows_a<R>(ra, rows_coef(), total == 1) && !el_rows_b<R>(ra, rows_coef(), total == 1))
               throw CudaError("internal: fused elastic rows for an unsupported length", MEU_ERR_UNSUPPORTED);
           });
@@ -1020,7 +1024,6 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
       elz_q_checked = elz_blocks > 0;
       if (h_ctl->status) throw CudaError("newfac is too small ... trouble converging", h_ctl->status);
       if (h_ctl->done) break;
-      cfac = h_ctl->cfac;
     }
   }
   last_iters = total;

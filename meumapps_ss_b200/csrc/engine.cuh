@@ -406,7 +406,7 @@ class Engine : public EngineBase {
   ElxCoef<R> el_prop_r{};  // the same in the field precision (fused row kernel)
   ElenProp en_prop{};  // proportional-moduli energy coefficients (host-built)
   // the instantiation of the proportional kernels for this stiffness form
-  void (*fn_el_x)(ElxProp, int64_t, const R*, const R*, R*, double, int*) = nullptr;
+  void (*fn_el_x)(ElxProp, int64_t, const R*, const R*, R*, const double*, int*) = nullptr;
   void (*fn_elener)(ElenProp, int64_t, const R*, const R*, const R*, R*, R*, int, int, double*, int*) = nullptr;
   size_t sm_el_x = 0, sm_elener = 0;  // their dynamic shared memory (prefetch tiles)
   bool el_ortho_gen = false;          // general moduli: C0 and every phase's compliance in that pattern
@@ -418,6 +418,11 @@ class Engine : public EngineBase {
   // the 3-D transform
   bool kks_axis = false;
   int kks_lap = 0;
+  // FP32 KKS with several variants: the n_tilda projection (Multi_MEUMAPPS.f:824-841) counts the
+  // variants with phi > 0, and in FP32 the transforms' rounding decides that sign wherever phi is
+  // within about 1e-8 of 0.  Any other order of operations moves a few voxels per million and step
+  // by up to 2e-3, so these decks keep the separate passes on their own radix plans.
+  bool keep_rounding = false;
   bool noise_live = false;            // phi_noise may be nonzero
   bool el_state = false;              // heterogeneous elasticity keeps a state between steps
   C* es = nullptr;

@@ -286,23 +286,23 @@ static bool dispatch_len(int L, int pv, F&& go) {
 }
 
 template <typename R>
-static bool rows_s(bool fwd, int L, int pv, int nf, int64_t nrows, const void* in, const void* out, const void* tw,
+static bool rows_s(bool fwd, bool mix, int L, int pv, int nf, int64_t nrows, const void* in, const void* out, const void* tw,
                    const void* post, cudaStream_t st) {
   auto go = [&](auto Lc, auto Pc) {
     return rows_launch<R, decltype(Lc)::value, decltype(Pc)::value>(fwd, nf, nrows, in, out, tw, post, st);
   };
-  return dispatch_len(L, pv, go) || rows_mix<R>(fwd, L, nf, nrows, in, out, tw, post, st);
+  return dispatch_len(L, pv, go) || (mix && rows_mix<R>(fwd, L, nf, nrows, in, out, tw, post, st));
 }
 
 template <typename R, bool FWD>
-static bool cols_s(int L, int pv, int ct, int nf, int outer, int inner, int64_t ostride, const PtrList<cplx<R>>& buf,
+static bool cols_s(bool mix, int L, int pv, int ct, int nf, int outer, int inner, int64_t ostride, const PtrList<cplx<R>>& buf,
                    const void* tw, R scale, cudaStream_t st) {
   auto go = [&](auto Lc, auto Pc) {
     constexpr int LL = decltype(Lc)::value, PV = decltype(Pc)::value, TM1 = col_tile_s<R>(LL);
     return ct == 2 ? cols_launch<R, FWD, LL, 2 * TM1, PV>(nf, outer, inner, ostride, buf, tw, scale, st)
                    : cols_launch<R, FWD, LL, TM1, PV>(nf, outer, inner, ostride, buf, tw, scale, st);
   };
-  return dispatch_len(L, pv, go) || cols_mix<R, FWD>(L, nf, outer, inner, ostride, buf, tw, scale, st);
+  return dispatch_len(L, pv, go) || (mix && cols_mix<R, FWD>(L, nf, outer, inner, ostride, buf, tw, scale, st));
 }
 
 static inline int col_tile(int L, bool fp64) {
@@ -337,7 +337,7 @@ void FFT3::forward_x(const PtrList<const R>& in, const PtrList<cplx<R>>& out, in
   set_smem<R>((const void*)k_rows_r2c<R>, sm);
   dim3 g((unsigned)((nrows + rpb - 1) / rpb), nf);
   { HookScope hs_(hook, "fft_x_r2c", (double)nf * (n3() * sizeof(R) + nk() * sizeof(C)), st);
-  if (!rows_s<R>(true, Lx, pv, nf, nrows, &in, &out, px.tw, post_tw, st))
+  if (!rows_s<R>(true, mix, Lx, pv, nf, nrows, &in, &out, px.tw, post_tw, st))
     k_rows_r2c<R><<<g, 256, sm, st>>>(in, out, nx, nrows, px, (const C*)post_tw); }
   MEU_CHECK_LAUNCH();
 }
@@ -357,12 +357,12 @@ void FFT3::pass_y(const PtrList<cplx<R>>& buf, int nf, bool fwd, cudaStream_t st
   const dim3 g2((unsigned)(nz * ((nxh + tm - 1) / tm)), nf);
   HookScope hs_(hook, fwd ? "fft_y_fwd" : "fft_y_inv", 2.0 * nf * nk() * sizeof(C), st);
   if (fwd) {
-    if (!cols_s<R, true>(ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, buf, py.tw, (R)1, st)) {
+    if (!cols_s<R, true>(mix, ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, buf, py.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, true>, s2);
       k_cols<R, true><<<g2, 256, s2, st>>>(buf, buf, nxh, (int64_t)ny * nxh, tm, py, (R)1);
     }
   } else {
-    if (!cols_s<R, false>(ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, buf, py.tw, (R)1, st)) {
+    if (!cols_s<R, false>(mix, ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, buf, py.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, false>, s2);
       k_cols<R, false><<<g2, 256, s2, st>>>(buf, buf, nxh, (int64_t)ny * nxh, tm, py, (R)1);
     }
@@ -381,12 +381,12 @@ void FFT3::pass_z(const PtrList<cplx<R>>& buf, int nf, bool fwd, cudaStream_t st
   HookScope hs_(hook, fwd ? "fft_z_fwd" : "fft_z_inv", 2.0 * nf * nk() * sizeof(C), st);
   if (fwd) {
     const R scale = (R)(1.0 / ((double)nx * ny * nz));
-    if (!cols_s<R, true>(nz, pv, ct, nf, 1, inner, 0, buf, pz.tw, scale, st)) {
+    if (!cols_s<R, true>(mix, nz, pv, ct, nf, 1, inner, 0, buf, pz.tw, scale, st)) {
       set_smem<R>((const void*)k_cols<R, true>, s3);
       k_cols<R, true><<<g3, 256, s3, st>>>(buf, buf, inner, 0, tm, pz, scale);
     }
   } else {
-    if (!cols_s<R, false>(nz, pv, ct, nf, 1, inner, 0, buf, pz.tw, (R)1, st)) {
+    if (!cols_s<R, false>(mix, nz, pv, ct, nf, 1, inner, 0, buf, pz.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, false>, s3);
       k_cols<R, false><<<g3, 256, s3, st>>>(buf, buf, inner, 0, tm, pz, (R)1);
     }
@@ -418,7 +418,7 @@ void FFT3::inverse_x(const PtrList<cplx<R>>& in, const PtrList<R>& out, int nf, 
   for (int f = 0; f < MAXF; ++f) cin.p[f] = in.p[f];
   dim3 g((unsigned)((nrows + rpb - 1) / rpb), nf);
   { HookScope hs_(hook, "fft_x_c2r", (double)nf * (n3() * sizeof(R) + nk() * sizeof(C)), st);
-  if (!rows_s<R>(false, Lx, pv, nf, nrows, &cin, &out, px.tw, post_tw, st))
+  if (!rows_s<R>(false, mix, Lx, pv, nf, nrows, &cin, &out, px.tw, post_tw, st))
     k_rows_c2r<R><<<g, 256, sm, st>>>(cin, out, nx, nrows, px, (const C*)post_tw); }
   MEU_CHECK_LAUNCH();
 }

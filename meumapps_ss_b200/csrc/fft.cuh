@@ -335,6 +335,9 @@ class FFT3 {
   // columns per block of the compile-time column kernels: ct = 1 about 32 KB of tile,
   // ct = 2 twice as many columns (longer contiguous runs, fewer blocks per SM)
   int ct = 1;
+  // compile-time kernels for the lengths with factors 3 (else their run-time plan, whose
+  // rounding differs: see Engine::keep_rounding)
+  bool mix = true;
   LaunchHook* hook = nullptr;
   const void* post_tw;  // cplx<R>[nx/2+1]: exp(-2 pi i k / nx)
   bool fp64;

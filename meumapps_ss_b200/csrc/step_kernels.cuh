@@ -235,7 +235,9 @@ __global__ void __launch_bounds__(256) k_el_zeroth(const DevConst* __restrict__ 
 // mix is inverted as a 3x3 block and three shears and the zero entries are skipped.
 template <typename R, bool ORTHO = false>
 __global__ void __launch_bounds__(256, ORTHO ? 3 : 1) k_el_x(const DevConst* __restrict__ Kp, const R* __restrict__ pphi,
-                                              const R* __restrict__ strain, R* __restrict__ xs, double cfac, int* err) {
+                                              const R* __restrict__ strain, R* __restrict__ xs,
+                                              const double* __restrict__ cfac_p, int* err) {
+  const double cfac = cfac_p ? *cfac_p : 1.0;
   const DevConst& K = *Kp;
   const meu_params& p = K.p;
   const int64_t n3 = K.n3;
@@ -326,7 +328,8 @@ __device__ __forceinline__ void pf_wait_prev() { asm volatile("cp.async.wait_gro
 template <typename R, bool ORTHO, bool VEC>
 __global__ void __launch_bounds__(PF_TILE, 4) k_el_x_prop(const __grid_constant__ ElxProp E, int64_t n3,
                                                           const R* __restrict__ pphi, const R* __restrict__ strain,
-                                                          R* __restrict__ xs, double cfac, int* err) {
+                                                          R* __restrict__ xs, const double* __restrict__ cfac_p, int* err) {
+  const double cfac = cfac_p ? *cfac_p : 1.0;
   constexpr int NV = MEU_MAX_VAR;
   const int V = E.nvar;
   const int NF = 6 + V;

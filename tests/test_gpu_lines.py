@@ -79,3 +79,35 @@ def test_kks_box_matches_oracle(oracle, nvar, numel, box):
     assert np.max(np.abs(ug - uo)) <= 1e-9 * np.max(np.abs(uo))
     for k in ("fint", "fch", "elen"):
         assert np.max(np.abs(d[k] - do[k])) <= 1e-9 * np.max(np.abs(do[k])), k
+
+
+def test_kks_off_diagonal_gradient_tensor_matches_oracle(oracle):
+    # gradient tensors with off-diagonal entries take the kappa-Laplacian through 3-D spectra
+    _, p, cons, phi = kks_case(24, 3, 4, ny=16, nz=18 * 2)
+    for v in range(3):
+        g = p.grad_coeff[v][0]
+        for i in (1, 3):
+            p.grad_coeff[v][i] = 0.2 * g
+        p.grad_coeff[v][5] = -0.1 * g
+    rng = np.random.default_rng(5)
+    phi = np.clip(phi + 0.2 * rng.uniform(0, 1, phi.shape) * (rng.uniform(size=phi.shape) > 0.2), 0.0, 1.0)
+    o = oracle.OracleSim(p)
+    o.set_fields(cons, phi)
+    o.run(3)
+    co, fo, _, _ = o.get_fields()
+    _, (cg, fg, _, _) = _run(p, cons, phi, 3)
+    assert np.max(np.abs(cg - co)) <= 1e-10 and np.max(np.abs(fg - fo)) <= 1e-10
+
+
+def test_kks_fp32_one_variant_against_fp64():
+    # the one-variant FP32 deck takes every fused path; bound as for the boxes above
+    _, p, cons, phi = kks_case(36, 1, 4, ny=24, nz=32)
+    rng = np.random.default_rng(9)
+    phi = np.clip(phi + 0.2 * rng.uniform(0, 1, phi.shape), 0.0, 1.0)
+    _, (c64, f64, _, _) = _run(p, cons, phi, 2)
+    q = p.copy()
+    q.precision = P.PREC_F32
+    _, (c32, f32, _, _) = _run(q, cons, phi, 2)
+    bound = 64 * 2.0 ** -24
+    assert np.linalg.norm(c32 - c64) <= bound * np.linalg.norm(c64)
+    assert np.linalg.norm(f32 - f64) <= bound * np.linalg.norm(f64)
