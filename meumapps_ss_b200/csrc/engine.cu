@@ -365,6 +365,20 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
   fft->mix = !keep_rounding;
   el_fused_rows = el_state && !keep_rounding && el_rows_ok(p.nx) && (hK.prop_moduli || el_ortho_gen);
   if (p.model == MEU_MODEL_KKS) {
+    KksPar& Q = kks_par;
+    for (int v = 0; v < V; ++v)
+      for (int i = 0; i < 9; ++i) Q.grad[v][i] = p.grad_coeff[v][i];
+    memcpy(Q.gparams, p.gparams, sizeof(Q.gparams));
+    memcpy(Q.wellph, p.wellph, sizeof(Q.wellph));
+    memcpy(Q.zconst, hK.zconst, sizeof(Q.zconst));
+    memcpy(Q.zr_const, hK.zr_const, sizeof(Q.zr_const));
+    memcpy(Q.ph_lo, hK.ph_lo, sizeof(Q.ph_lo));
+    memcpy(Q.ph_hi, hK.ph_hi, sizeof(Q.ph_hi));
+    Q.nvar = V;
+    Q.numel = E;
+    Q.numph = p.numph;
+    Q.zdim = hK.zdim;
+    Q.n3 = n3;
     kks_axis = !keep_rounding && axis_ok(p.nx) && axis_ok(p.ny) && axis_ok(p.nz);
     // off-diagonal gradient coefficients below the rounding of the diagonal's (a rotated
     // isotropic tensor) do not need the 3-D route
@@ -1092,13 +1106,18 @@ void Engine<R>::kks_step(meu_diag* d) {
   }
   // local driving force (:619-845)
   {
-    // compile-time phase and solute counts for the common decks (composition solve in registers)
+    // compile-time counts for the common decks (composition solve and variants in registers)
     auto kp = k_kks_point<R>;
-    if (P.numph == 2 && P.numel == 1) kp = k_kks_point<R, 2, 1>;
-    else if (P.numph == 3 && P.numel == 1) kp = k_kks_point<R, 3, 1>;
-    else if (P.numph == 2 && P.numel == 2) kp = k_kks_point<R, 2, 2>;
+    if (P.numph == 2 && P.numel == 1) {
+      kp = V == 1 ? k_kks_point<R, 2, 1, 1> : V == 3 ? k_kks_point<R, 2, 1, 3> : V == 12 ? k_kks_point<R, 2, 1, 12>
+                                                                                         : k_kks_point<R, 2, 1>;
+    } else if (P.numph == 3 && P.numel == 1) {
+      kp = k_kks_point<R, 3, 1>;
+    } else if (P.numph == 2 && P.numel == 2) {
+      kp = V == 1 ? k_kks_point<R, 2, 2, 1> : V == 3 ? k_kks_point<R, 2, 2, 3> : k_kks_point<R, 2, 2>;
+    }
     KLAUNCH("kks_point", (double)(7 * V + 4 * E) * n3 * sizeof(R),
-            kp<<<RED_BLOCKS, RED_THREADS, 0, st>>>(dK, phi, c, wr, pphi, fd, fc, partials, d_err));
+            kp<<<RED_BLOCKS, RED_THREADS, 0, st>>>(kks_par, phi, c, wr, pphi, fd, fc, partials, d_err));
   }
   // elasticity (:851-880); on the row path elener writes the TDGL right-hand side into fd
   last_iters = 0;

@@ -423,6 +423,7 @@ class Engine : public EngineBase {
   // within about 1e-8 of 0.  Any other order of operations moves a few voxels per million and step
   // by up to 2e-3, so these decks keep the separate passes on their own radix plans.
   bool keep_rounding = false;
+  KksPar kks_par{};
   bool noise_live = false;            // phi_noise may be nonzero
   bool el_state = false;              // heterogeneous elasticity keeps a state between steps
   C* es = nullptr;

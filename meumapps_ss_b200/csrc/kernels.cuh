@@ -46,6 +46,16 @@ struct DevConst {
   int c_shift;
 };
 
+// KKS: the constants of the driving force, by value (the products read them from the parameter bank
+// instead of reloading them for every voxel).
+struct KksPar {
+  double grad[MEU_MAX_VAR][9], gparams[MEU_MAX_PH][MEU_MAX_GP], wellph[MEU_MAX_PH];
+  double zconst[144], zr_const[12];
+  int ph_lo[MEU_MAX_PH + 1], ph_hi[MEU_MAX_PH + 1];
+  int nvar, numel, numph, zdim;
+  int64_t n3;
+};
+
 enum RedQ : int {
   Q_FCH = 0, Q_FW, Q_FINT, Q_ELEN, Q_CMIN, Q_CMAX, Q_PHIMAX, Q_SOLID, Q_CSUM0,
   // gradient energy of the fields a step produces (the next step's start-of-step value)

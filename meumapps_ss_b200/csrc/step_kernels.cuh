@@ -60,46 +60,67 @@ __global__ void __launch_bounds__(256) k_kks_lap(const DevConst* __restrict__ Kp
 
 // ------------------------------------------------- KKS: local driving force
 // Multi_MEUMAPPS.f:634-845 per voxel.  g4 = [gx_v, gy_v, gz_v, kds_v] per v.
-// Fields in R; the local solve and the energies in FP64.  NPH, NEL > 0: the phase and
-// solute counts are compile-time (the common decks), so the zdim x zdim composition
-// system and its inverse live in registers; 0, 0: any counts, arrays sized for the
-// largest system (local memory).
-template <typename R, int NPH = 0, int NEL = 0>
-__global__ void __launch_bounds__(RED_THREADS) k_kks_point(const DevConst* __restrict__ Kp, const R* __restrict__ phi,
-                                                           const R* __restrict__ cons, const R* __restrict__ g4,
-                                                           R* __restrict__ pphi, R* __restrict__ fdiff,
-                                                           R* __restrict__ fc, double* partials, int* err) {
-  const DevConst& K = *Kp;
-  const meu_params& p = K.p;
+// Fields in R; the local solve and the energies in FP64.  NPH, NEL > 0: the phase and solute
+// counts are compile-time (the common decks), so the zdim x zdim composition system and its
+// inverse live in registers; NV > 0: the variant count too, so the per-variant values do and the
+// voxel's loads are all in flight together (KKS 128^3, 3 variants: 231 -> 125 us).  0: any counts,
+// arrays sized for the largest system (local memory).
+template <typename R, int NPH = 0, int NEL = 0, int NV = 0>
+__global__ void __launch_bounds__(RED_THREADS, NV > 0 && NV <= 4 ? 2 : 1)
+    k_kks_point(const __grid_constant__ KksPar p, const R* __restrict__ phi, const R* __restrict__ cons,
+                const R* __restrict__ g4, R* __restrict__ pphi, R* __restrict__ fdiff, R* __restrict__ fc,
+                double* partials, int* err) {
   constexpr bool FIX = NPH > 0 && NEL > 0;
   constexpr int ZM = FIX ? NPH * NEL : 12;  // largest zdim the arrays hold
-  const int V = p.nvar, numel = FIX ? NEL : p.numel, numph = FIX ? NPH : p.numph, zdim = FIX ? ZM : K.zdim;
-  const int64_t n3 = K.n3;
+  constexpr int VM = NV > 0 ? NV : MEU_MAX_VAR;
+  constexpr int UN = NV > 0 ? NV : 1;  // the variant loops unroll when their length is known
+  const int V = NV > 0 ? NV : p.nvar, numel = FIX ? NEL : p.numel, numph = FIX ? NPH : p.numph, zdim = FIX ? ZM : p.zdim;
+  const int64_t n3 = p.n3;
   double fch = 0, fw = 0, fint = 0;
   for (int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < n3; id += (int64_t)gridDim.x * blockDim.x) {
-    double Pph[MEU_MAX_PH], Gph[MEU_MAX_PH], Ppr[MEU_MAX_VAR], fgrad[MEU_MAX_VAR], ph[MEU_MAX_VAR];
+    double Pph[MEU_MAX_PH], Gph[MEU_MAX_PH], Ppr[VM], fgrad[VM], ph[VM], kds[VM], gr[NV > 0 ? NV : 1][3], cin[MEU_MAX_EL];
     for (int n = 0; n < MEU_MAX_PH; ++n) { Pph[n] = 0; Gph[n] = 0; }
+#pragma unroll UN
     for (int v = 0; v < V; ++v) ph[v] = (double)phi[v * n3 + id];
-    for (int n = 2; n <= numph; ++n)
-      for (int v = K.ph_lo[n]; v < K.ph_hi[n]; ++v) {
-        const double fi = ph[v], fi_sq = fi * fi;
-        const double pl = fi_sq * fi * (6.0 * fi_sq - 15.0 * fi + 10.0);
-        pphi[v * n3 + id] = (R)pl;
-        Ppr[v] = 30.0 * fi_sq * (fi_sq - 2.0 * fi + 1.0);
-        Pph[0] += pl;
-        Pph[n - 1] += pl;
-        Gph[n - 1] += fi_sq * (1.0 - fi) * (1.0 - fi);
-        for (int u = 0; u < V; ++u)
-          if (u != v) Gph[0] += fi_sq * ph[u] * ph[u];
+    for (int e = 0; e < numel; ++e) cin[e] = (double)cons[e * n3 + id];
+    if (NV > 0) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) gr[v][d] = (double)g4[(4 * v + d) * n3 + id];
+        if (NV > 1) kds[v] = (double)g4[(4 * v + 3) * n3 + id];
       }
+    }
+    // with one precipitate phase every variant belongs to it
+    auto variants = [&](auto&& fn) {
+      if (NPH == 2) {
+#pragma unroll UN
+        for (int v = 0; v < V; ++v) fn(2, v);
+      } else {
+        for (int n = 2; n <= numph; ++n)
+          for (int v = p.ph_lo[n]; v < p.ph_hi[n]; ++v) fn(n, v);
+      }
+    };
+    variants([&](int n, int v) {
+      const double fi = ph[v], fi_sq = fi * fi;
+      const double pl = fi_sq * fi * (6.0 * fi_sq - 15.0 * fi + 10.0);
+      pphi[v * n3 + id] = (R)pl;
+      Ppr[v] = 30.0 * fi_sq * (fi_sq - 2.0 * fi + 1.0);
+      Pph[0] += pl;
+      Pph[n - 1] += pl;
+      Gph[n - 1] += fi_sq * (1.0 - fi) * (1.0 - fi);
+#pragma unroll UN
+      for (int u = 0; u < V; ++u)
+        if (u != v) Gph[0] += fi_sq * ph[u] * ph[u];
+    });
     Pph[0] = 1.0 - Pph[0];
     // interface compositions (:677-710)
     double Z[ZM * ZM], Zr[ZM], X[MEU_MAX_EL][MEU_MAX_PH], Gib[MEU_MAX_PH], MuC[MEU_MAX_EL];
-    for (int i = 0; i < zdim * zdim; ++i) Z[i] = K.zconst[i];
-    for (int i = 0; i < zdim; ++i) Zr[i] = K.zr_const[i];
+    for (int i = 0; i < zdim * zdim; ++i) Z[i] = p.zconst[i];
+    for (int i = 0; i < zdim; ++i) Zr[i] = p.zr_const[i];
     for (int e = 1; e <= numel; ++e) {
       const int i0 = zdim - numel + e;
-      Zr[i0 - 1] = (double)cons[(e - 1) * n3 + id];
+      Zr[i0 - 1] = cin[e - 1];
       for (int n = 1; n <= numph; ++n) Z[(i0 - 1) + (numph * (e - 1) + n - 1) * zdim] = Pph[n - 1];
     }
     set_err(err, invert_small<ZM>(Z, zdim, MEU_ERR_Z_SINGULAR));
@@ -124,29 +145,31 @@ __global__ void __launch_bounds__(RED_THREADS) k_kks_point(const DevConst* __res
     double fchloc = Pph[0] * Gib[0], fwloc = p.wellph[0] * Gph[0];
     double fcl[3 * MEU_MAX_EL];
     for (int i = 0; i < 3 * numel; ++i) fcl[i] = 0;
-    for (int n = 2; n <= numph; ++n) {
-      for (int v = K.ph_lo[n]; v < K.ph_hi[n]; ++v) {
-        const double* g = p.grad_coeff[v];
-        const double gx = (double)g4[(4 * v + 0) * n3 + id], gy = (double)g4[(4 * v + 1) * n3 + id];
-        const double gz = (double)g4[(4 * v + 2) * n3 + id];
-        const double term = g[0] * gx * gx + g[4] * gy * gy + g[8] * gz * gz + (g[3] + g[1]) * gx * gy +
-                            (g[6] + g[2]) * gx * gz + (g[7] + g[5]) * gy * gz;
-        fint += 0.5 * term;
-        const double fi = ph[v];
-        double termch = Gib[n - 1] - Gib[0];
-        for (int e = 0; e < numel; ++e) {
-          const double xd = X[e][0] - X[e][n - 1];
-          termch += MuC[e] * xd;
-          const double t = Ppr[v] * xd;
-          fcl[3 * e + 0] += t * gx;
-          fcl[3 * e + 1] += t * gy;
-          fcl[3 * e + 2] += t * gz;
-        }
-        double well = 2.0 * p.wellph[n - 1] * fi * (1.0 - fi) * (1.0 - 2.0 * fi);
-        for (int u = 0; u < V; ++u)
-          if (u != v) well += 4.0 * p.wellph[0] * fi * ph[u] * ph[u];
-        fgrad[v] = termch * Ppr[v] + well;
+    variants([&](int n, int v) {
+      const double* g = p.grad[v];
+      const double gx = NV > 0 ? gr[NV > 0 ? v : 0][0] : (double)g4[(4 * v + 0) * n3 + id];
+      const double gy = NV > 0 ? gr[NV > 0 ? v : 0][1] : (double)g4[(4 * v + 1) * n3 + id];
+      const double gz = NV > 0 ? gr[NV > 0 ? v : 0][2] : (double)g4[(4 * v + 2) * n3 + id];
+      const double term = g[0] * gx * gx + g[4] * gy * gy + g[8] * gz * gz + (g[3] + g[1]) * gx * gy +
+                          (g[6] + g[2]) * gx * gz + (g[7] + g[5]) * gy * gz;
+      fint += 0.5 * term;
+      const double fi = ph[v];
+      double termch = Gib[n - 1] - Gib[0];
+      for (int e = 0; e < numel; ++e) {
+        const double xd = X[e][0] - X[e][n - 1];
+        termch += MuC[e] * xd;
+        const double t = Ppr[v] * xd;
+        fcl[3 * e + 0] += t * gx;
+        fcl[3 * e + 1] += t * gy;
+        fcl[3 * e + 2] += t * gz;
       }
+      double well = 2.0 * p.wellph[n - 1] * fi * (1.0 - fi) * (1.0 - 2.0 * fi);
+#pragma unroll UN
+      for (int u = 0; u < V; ++u)
+        if (u != v) well += 4.0 * p.wellph[0] * fi * ph[u] * ph[u];
+      fgrad[v] = termch * Ppr[v] + well;
+    });
+    for (int n = 2; n <= numph; ++n) {
       fchloc += Pph[n - 1] * Gib[n - 1];
       fwloc += p.wellph[n - 1] * Gph[n - 1];
     }
@@ -154,15 +177,18 @@ __global__ void __launch_bounds__(RED_THREADS) k_kks_point(const DevConst* __res
     fw += fwloc;
     for (int i = 0; i < 3 * numel; ++i) fc[(int64_t)i * n3 + id] = (R)fcl[i];
     // n_tilda projection (:824-841)
+#pragma unroll UN
     for (int jv = 0; jv < V; ++jv) {
       double term11 = 0;
       int nt = 1;
-      if (ph[jv] > 0.0)
+      if (ph[jv] > 0.0) {
+#pragma unroll UN
         for (int iv = 0; iv < V; ++iv)
           if (ph[iv] > 0.0 && iv != jv) {
-            term11 += fgrad[iv] - (double)g4[(4 * iv + 3) * n3 + id];
+            term11 += fgrad[iv] - (NV > 1 ? kds[iv] : (double)g4[(4 * iv + 3) * n3 + id]);
             nt += 1;
           }
+      }
       fdiff[jv * n3 + id] = (R)(fgrad[jv] - term11 / (double)nt);
     }
   }
