@@ -398,8 +398,9 @@ void EnsembleT<R>::get_fields(int m, double* cons, double* phi, double* el_en) {
 template <typename R>
 void EnsembleT<R>::schedule(int m, int32_t* out) const {
   if (m < 0 || m >= members) throw CudaError("member index out of range", MEU_ERR_BADARG);
-  const LanSched& s = bk[bucket_of[m]].sched;
-  const int tm = s.tm ? s.tm : (sizeof(R) == 4 ? 16 : 8);
+  const auto& b = bk[bucket_of[m]];
+  const LanSched& s = b.sched;
+  const int tm = s.tm ? s.tm : lan_default_tm(b.N, b.V, sizeof(R) == 8);
   out[0] = s.pv;
   out[1] = s.ntp;
   out[2] = tm;

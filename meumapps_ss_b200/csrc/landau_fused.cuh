@@ -89,8 +89,21 @@ struct LanFusedArgs {
 // Schedule of the fused kernels: radix plan variant (fz::rplan), threads of the
 // plane kernels, column tile width (complex columns per column-kernel block).
 struct LanSched {
-  int pv = 0, ntp = 512, tm = 0;  // tm = 0: 16 columns (FP32) / 8 columns (FP64)
+  int pv = 0, ntp = 512, tm = 0;  // tm = 0: lan_default_tm
 };
+// Column tile of a handle that sets none.  The column kernels are bound by latency, so more and
+// smaller blocks win until a tile's runs in global memory (tm complex) get short.  Measured on the
+// default radix plan and plane threads, us per step:
+//  FP32 8 / 16 columns: 128^3 two variants 126 / 134, three 176 / 188, four 221 / 249; 64^3 two to
+//   four 33.9 / 40.0, 37.5 / 47.2, 44.8 / 52.8.  One variant keeps 16: a single grid gains at most
+//   9% (48^3), but the members of an ensemble fill the GPU anyway and lose 6% on average, and
+//   they run the schedule of single handles;
+//  FP64 4 / 8 columns: 32^3 two to four variants 20.6 / 21.5, 21.5 / 23.3, 23.5 / 28.1; 48^3 two to
+//   four 35.2 / 31.1, 37.9 / 44.4, 42.3 / 49.4; 64^3 and larger 8 (4 is 0 to 17% slower).
+inline int lan_default_tm(int N, int V, bool f64) {
+  if (f64) return (N <= 48 && V >= 3) || (N <= 32 && V >= 2) ? 4 : 8;
+  return V == 1 ? 16 : 8;
+}
 
 enum LanQ : int {
   LQ_FCH = Q_FCH, LQ_FINT = Q_FINT, LQ_ELEN = Q_ELEN, LQ_CMIN = Q_CMIN, LQ_CMAX = Q_CMAX, LQ_PHIMAX = Q_PHIMAX,
