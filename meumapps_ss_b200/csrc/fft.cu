@@ -295,14 +295,14 @@ static bool rows_s(bool fwd, bool mix, int L, int pv, int nf, int64_t nrows, con
 }
 
 template <typename R, bool FWD>
-static bool cols_s(bool mix, int L, int pv, int ct, int nf, int outer, int inner, int64_t ostride, const PtrList<cplx<R>>& buf,
-                   const void* tw, R scale, cudaStream_t st) {
+static bool cols_s(bool mix, int L, int pv, int ct, int nf, int outer, int inner, int64_t ostride,
+                   const PtrList<cplx<R>>& in, const PtrList<cplx<R>>& out, const void* tw, R scale, cudaStream_t st) {
   auto go = [&](auto Lc, auto Pc) {
     constexpr int LL = decltype(Lc)::value, PV = decltype(Pc)::value, TM1 = col_tile_s<R>(LL);
-    return ct == 2 ? cols_launch<R, FWD, LL, 2 * TM1, PV>(nf, outer, inner, ostride, buf, tw, scale, st)
-                   : cols_launch<R, FWD, LL, TM1, PV>(nf, outer, inner, ostride, buf, tw, scale, st);
+    return ct == 2 ? cols_launch<R, FWD, LL, 2 * TM1, PV>(nf, outer, inner, ostride, in, out, tw, scale, st)
+                   : cols_launch<R, FWD, LL, TM1, PV>(nf, outer, inner, ostride, in, out, tw, scale, st);
   };
-  return dispatch_len(L, pv, go) || (mix && cols_mix<R, FWD>(L, nf, outer, inner, ostride, buf, tw, scale, st));
+  return dispatch_len(L, pv, go) || (mix && cols_mix<R, FWD>(L, nf, outer, inner, ostride, in, out, tw, scale, st));
 }
 
 static inline int col_tile(int L, bool fp64) {
@@ -350,21 +350,21 @@ void FFT3::forward_cols(const PtrList<cplx<R>>& out, int nf, cudaStream_t st) co
 
 // y columns: outer = z, inner = nxh
 template <typename R>
-void FFT3::pass_y(const PtrList<cplx<R>>& buf, int nf, bool fwd, cudaStream_t st) const {
+void FFT3::pass_y(const PtrList<cplx<R>>& in, const PtrList<cplx<R>>& out, int nf, bool fwd, cudaStream_t st) const {
   using C = cplx<R>;
   const int tm = col_tile(ny, sizeof(R) == 8);
   const size_t s2 = (size_t)ny * tm * sizeof(C);
   const dim3 g2((unsigned)(nz * ((nxh + tm - 1) / tm)), nf);
   HookScope hs_(hook, fwd ? "fft_y_fwd" : "fft_y_inv", 2.0 * nf * nk() * sizeof(C), st);
   if (fwd) {
-    if (!cols_s<R, true>(mix, ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, buf, py.tw, (R)1, st)) {
+    if (!cols_s<R, true>(mix, ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, in, out, py.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, true>, s2);
-      k_cols<R, true><<<g2, 256, s2, st>>>(buf, buf, nxh, (int64_t)ny * nxh, tm, py, (R)1);
+      k_cols<R, true><<<g2, 256, s2, st>>>(in, out, nxh, (int64_t)ny * nxh, tm, py, (R)1);
     }
   } else {
-    if (!cols_s<R, false>(mix, ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, buf, py.tw, (R)1, st)) {
+    if (!cols_s<R, false>(mix, ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, in, out, py.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, false>, s2);
-      k_cols<R, false><<<g2, 256, s2, st>>>(buf, buf, nxh, (int64_t)ny * nxh, tm, py, (R)1);
+      k_cols<R, false><<<g2, 256, s2, st>>>(in, out, nxh, (int64_t)ny * nxh, tm, py, (R)1);
     }
   }
   MEU_CHECK_LAUNCH();
@@ -381,12 +381,12 @@ void FFT3::pass_z(const PtrList<cplx<R>>& buf, int nf, bool fwd, cudaStream_t st
   HookScope hs_(hook, fwd ? "fft_z_fwd" : "fft_z_inv", 2.0 * nf * nk() * sizeof(C), st);
   if (fwd) {
     const R scale = (R)(1.0 / ((double)nx * ny * nz));
-    if (!cols_s<R, true>(mix, nz, pv, ct, nf, 1, inner, 0, buf, pz.tw, scale, st)) {
+    if (!cols_s<R, true>(mix, nz, pv, ct, nf, 1, inner, 0, buf, buf, pz.tw, scale, st)) {
       set_smem<R>((const void*)k_cols<R, true>, s3);
       k_cols<R, true><<<g3, 256, s3, st>>>(buf, buf, inner, 0, tm, pz, scale);
     }
   } else {
-    if (!cols_s<R, false>(mix, nz, pv, ct, nf, 1, inner, 0, buf, pz.tw, (R)1, st)) {
+    if (!cols_s<R, false>(mix, nz, pv, ct, nf, 1, inner, 0, buf, buf, pz.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, false>, s3);
       k_cols<R, false><<<g3, 256, s3, st>>>(buf, buf, inner, 0, tm, pz, (R)1);
     }
@@ -435,8 +435,8 @@ template void FFT3::forward_x<float>(const PtrList<const float>&, const PtrList<
 template void FFT3::forward_x<double>(const PtrList<const double>&, const PtrList<double2>&, int, cudaStream_t) const;
 template void FFT3::inverse_x<float>(const PtrList<float2>&, const PtrList<float>&, int, cudaStream_t) const;
 template void FFT3::inverse_x<double>(const PtrList<double2>&, const PtrList<double>&, int, cudaStream_t) const;
-template void FFT3::pass_y<float>(const PtrList<float2>&, int, bool, cudaStream_t) const;
-template void FFT3::pass_y<double>(const PtrList<double2>&, int, bool, cudaStream_t) const;
+template void FFT3::pass_y<float>(const PtrList<float2>&, const PtrList<float2>&, int, bool, cudaStream_t) const;
+template void FFT3::pass_y<double>(const PtrList<double2>&, const PtrList<double2>&, int, bool, cudaStream_t) const;
 template void FFT3::pass_z<float>(const PtrList<float2>&, int, bool, cudaStream_t) const;
 template void FFT3::pass_z<double>(const PtrList<double2>&, int, bool, cudaStream_t) const;
 

@@ -318,13 +318,17 @@ class FFT3 {
   template <typename R>
   void inverse_cols(const PtrList<cplx<R>>& in, int nf, cudaStream_t st) const;
   // single passes: x forward (real in, spectrum rows out), x inverse (spectrum rows
-  // in, used as scratch; real out), y and z in place
+  // in, used as scratch; real out), y (in place or not) and z in place
   template <typename R>
   void forward_x(const PtrList<const R>& in, const PtrList<cplx<R>>& out, int nf, cudaStream_t st) const;
   template <typename R>
   void inverse_x(const PtrList<cplx<R>>& in, const PtrList<R>& out, int nf, cudaStream_t st) const;
   template <typename R>
-  void pass_y(const PtrList<cplx<R>>& buf, int nf, bool fwd, cudaStream_t st) const;
+  void pass_y(const PtrList<cplx<R>>& in, const PtrList<cplx<R>>& out, int nf, bool fwd, cudaStream_t st) const;
+  template <typename R>
+  void pass_y(const PtrList<cplx<R>>& buf, int nf, bool fwd, cudaStream_t st) const {
+    pass_y<R>(buf, buf, nf, fwd, st);
+  }
   template <typename R>
   void pass_z(const PtrList<cplx<R>>& buf, int nf, bool fwd, cudaStream_t st) const;
 

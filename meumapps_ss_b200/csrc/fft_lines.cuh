@@ -192,13 +192,13 @@ bool rows_launch(bool fwd, int nf, int64_t nrows, const void* in, const void* ou
   return true;
 }
 template <typename R, bool FWD, int LL, int TM, int PV>
-bool cols_launch(int nf, int outer, int inner, int64_t ostride, const PtrList<cplx<R>>& buf, const void* tw, R scale,
-                 cudaStream_t st) {
+bool cols_launch(int nf, int outer, int inner, int64_t ostride, const PtrList<cplx<R>>& in,
+                 const PtrList<cplx<R>>& out, const void* tw, R scale, cudaStream_t st) {
   using C = cplx<R>;
   const size_t sm = (size_t)LL * TM * sizeof(C);
   set_smem<R>((const void*)k_cols_s<R, FWD, LL, TM, PV>, sm);
   const dim3 g((unsigned)(outer * ((inner + TM - 1) / TM)), nf);
-  k_cols_s<R, FWD, LL, TM, PV><<<g, 256, sm, st>>>(buf, buf, inner, ostride, (const C*)tw, scale);
+  k_cols_s<R, FWD, LL, TM, PV><<<g, 256, sm, st>>>(in, out, inner, ostride, (const C*)tw, scale);
   return true;
 }
 // lengths with factors 3 (radix plan 3); false when L has no such kernel
@@ -206,7 +206,7 @@ template <typename R>
 bool rows_mix(bool fwd, int L, int nf, int64_t nrows, const void* in, const void* out, const void* tw,
               const void* post, cudaStream_t st);
 template <typename R, bool FWD>
-bool cols_mix(int L, int nf, int outer, int inner, int64_t ostride, const PtrList<cplx<R>>& buf, const void* tw,
-              R scale, cudaStream_t st);
+bool cols_mix(int L, int nf, int outer, int inner, int64_t ostride, const PtrList<cplx<R>>& in,
+              const PtrList<cplx<R>>& out, const void* tw, R scale, cudaStream_t st);
 
 }  // namespace meu

@@ -3,6 +3,8 @@
 
 namespace meu {
 template bool rows_mix<float>(bool, int, int, int64_t, const void*, const void*, const void*, const void*, cudaStream_t);
-template bool cols_mix<float, true>(int, int, int, int, int64_t, const PtrList<cplx<float>>&, const void*, float, cudaStream_t);
-template bool cols_mix<float, false>(int, int, int, int, int64_t, const PtrList<cplx<float>>&, const void*, float, cudaStream_t);
+template bool cols_mix<float, true>(int, int, int, int, int64_t, const PtrList<cplx<float>>&,
+                                   const PtrList<cplx<float>>&, const void*, float, cudaStream_t);
+template bool cols_mix<float, false>(int, int, int, int, int64_t, const PtrList<cplx<float>>&,
+                                   const PtrList<cplx<float>>&, const void*, float, cudaStream_t);
 }  // namespace meu

@@ -3,6 +3,8 @@
 
 namespace meu {
 template bool rows_mix<double>(bool, int, int, int64_t, const void*, const void*, const void*, const void*, cudaStream_t);
-template bool cols_mix<double, true>(int, int, int, int, int64_t, const PtrList<cplx<double>>&, const void*, double, cudaStream_t);
-template bool cols_mix<double, false>(int, int, int, int, int64_t, const PtrList<cplx<double>>&, const void*, double, cudaStream_t);
+template bool cols_mix<double, true>(int, int, int, int, int64_t, const PtrList<cplx<double>>&,
+                                   const PtrList<cplx<double>>&, const void*, double, cudaStream_t);
+template bool cols_mix<double, false>(int, int, int, int, int64_t, const PtrList<cplx<double>>&,
+                                   const PtrList<cplx<double>>&, const void*, double, cudaStream_t);
 }  // namespace meu

@@ -85,9 +85,14 @@ void planes_forward(meu_slab_fft* h, const void* real, void* send, cudaStream_t 
   PtrList<const R> a{};
   PtrList<C> b{};
   a.p[0] = (const R*)real;
-  b.p[0] = (C*)h->spec;
+  // one rank: the send buffer is the planes' spectrum (P = 1 packs nothing), transformed in it
+  b.p[0] = (C*)(h->P == 1 ? send : h->spec);
   h->planes->forward_x<R>(a, b, 1, st);
   h->planes->pass_y<R>(b, 1, true, st);
+  if (h->P == 1) {
+    h->launches += 2;
+    return;
+  }
   const int64_t n = (int64_t)h->P * h->nzl * h->nyl * h->nxh;
   k_slab_pack<C, R><<<grid_for(n, 256), 256, 0, st>>>((const C*)h->spec, (C*)send, h->P, h->nzl, h->ny, h->nyl,
                                                        h->nxh, (R)(1.0 / h->P));
@@ -97,6 +102,18 @@ void planes_forward(meu_slab_fft* h, const void* real, void* send, cudaStream_t 
 template <typename R>
 void planes_inverse(meu_slab_fft* h, const void* recv, void* real, cudaStream_t st) {
   using C = cplx<R>;
+  if (h->P == 1) {
+    // one rank: the receive buffer is the planes' spectrum; the y pass reads it there
+    PtrList<C> r{}, b{};
+    PtrList<R> o{};
+    r.p[0] = (C*)recv;
+    b.p[0] = (C*)h->spec;
+    o.p[0] = (R*)real;
+    h->planes->pass_y<R>(r, b, 1, false, st);
+    h->planes->inverse_x<R>(b, o, 1, st);
+    h->launches += 2;
+    return;
+  }
   const int64_t n = (int64_t)h->P * h->nzl * h->nyl * h->nxh;
   k_slab_unpack<C><<<grid_for(n, 256), 256, 0, st>>>((const C*)recv, (C*)h->spec, h->P, h->nzl, h->ny, h->nyl,
                                                      h->nxh);

@@ -79,7 +79,8 @@ class SlabFFT:
         g = self.geo
         self.kslab_shape = (nz, g["nyl"], g["nxh"])
         self.real_shape = (g["nzl"], ny, nx)
-        self._buf = torch.empty(self.kslab_shape, dtype=self.cdtype, device=self.device)
+        # send / receive buffer of the all-to-all
+        self._buf = torch.empty(self.kslab_shape, dtype=self.cdtype, device=self.device) if nranks > 1 else None
 
     def close(self) -> None:
         if getattr(self, "h", None):
@@ -108,10 +109,13 @@ class SlabFFT:
         if tuple(real.shape) != self.real_shape or real.dtype != self.rdtype or not real.is_contiguous():
             raise ValueError(f"real slab must be a contiguous {self.rdtype} tensor of shape {self.real_shape}")
         st = self._stream()
-        self._check(lib().meu_slab_fft_forward_planes(self.h, C.c_void_p(real.data_ptr()),
-                                                      C.c_void_p(self._buf.data_ptr()), st))
         kslab = torch.empty(self.kslab_shape, dtype=self.cdtype, device=self.device)
-        exchange(self._buf, kslab, self.group)
+        # one rank exchanges nothing: its send buffer is the k-slab
+        send = kslab if self.nranks == 1 else self._buf
+        self._check(lib().meu_slab_fft_forward_planes(self.h, C.c_void_p(real.data_ptr()),
+                                                      C.c_void_p(send.data_ptr()), st))
+        if self.nranks > 1:
+            exchange(send, kslab, self.group)
         self._check(lib().meu_slab_fft_forward_columns(self.h, C.c_void_p(kslab.data_ptr()), st))
         return kslab
 
@@ -124,8 +128,10 @@ class SlabFFT:
             raise ValueError(f"k-slab must be a contiguous {self.cdtype} tensor of shape {self.kslab_shape}")
         st = self._stream()
         self._check(lib().meu_slab_fft_inverse_columns(self.h, C.c_void_p(kslab.data_ptr()), st))
-        exchange(kslab, self._buf, self.group)
+        recv = kslab if self.nranks == 1 else self._buf
+        if self.nranks > 1:
+            exchange(kslab, recv, self.group)
         real = torch.empty(self.real_shape, dtype=self.rdtype, device=self.device)
-        self._check(lib().meu_slab_fft_inverse_planes(self.h, C.c_void_p(self._buf.data_ptr()),
+        self._check(lib().meu_slab_fft_inverse_planes(self.h, C.c_void_p(recv.data_ptr()),
                                                       C.c_void_p(real.data_ptr()), st))
         return real
