@@ -266,10 +266,31 @@ void Engine<R>::adjoint(int T, int K, const double* cons_tgt, const double* phi_
   int nb[Q_TOTAL];
   const int64_t step0 = step;
   auto homog_at = [&](int64_t s) { return (P.elastic != MEU_ELAST_NONE && s >= P.elastep0) ? 1 : 0; };
-  // ---- forward, in place, with checkpoints every K steps
+  // ---- forward, in place, with checkpoints every K steps.  The last segment runs out of place into
+  // the per-step buffers with theta^ and phi recorded, as the reverse sweep would recompute it:
+  // that segment needs no recomputation.
   LanFusedArgs<R> fa = fused_args();
   fa.energy = 0;
   int up_homog = -1;
+  const int last0 = (nck - 1) * K;
+  // record j of a segment starting at step i0 from checkpoint seg
+  auto record = [&](int seg, int j) {
+    LanFusedArgs<R> r = fa;
+    r.homog = homog_at(step0 + (int64_t)seg * K + j);
+    r.eta = j == 0 ? B.ck_eta[seg] : B.s_eta[j];
+    r.c = j == 0 ? B.ck_c[seg] : B.s_c[j];
+    r.Keta = j == 0 ? B.ck_keta[seg] : B.s_keta[j];
+    r.Kc = j == 0 ? B.ck_kc[seg] : B.s_kc[j];
+    r.eta_next = B.s_eta[j + 1];
+    r.c_next = B.s_c[j + 1];
+    r.Keta_out = B.s_keta[j + 1];
+    r.Kc_out = B.s_kc[j + 1];
+    r.rec_phi = B.s_phi[j];
+    r.rec_theta = B.s_theta[j];
+    return r;
+  };
+  MEU_CUDA(cudaStreamSynchronize(st));  // hRec may still be in flight from an earlier call
+  for (int j = 0; j < T - last0; ++j) B.hRec[j] = record(nck - 1, j);
   for (int i = 0; i < T; ++i) {
     if (i % K == 0) {
       const int s = i / K;
@@ -280,23 +301,37 @@ void Engine<R>::adjoint(int T, int K, const double* cons_tgt, const double* phi_
       // theta^ of these fields, as the previous forward step's PI wrote it: the recomputed
       // segment then starts from the same numbers instead of transforming theta afresh
       B.ck_has_theta[s] = theta_ready ? 1 : 0;
-      if (theta_ready) MEU_CUDA(cudaMemcpyAsync(B.ck_theta[s], sp, sizeof(C) * V * nk, cudaMemcpyDeviceToDevice, st));
+      if (theta_ready && s < nck - 1)
+        MEU_CUDA(cudaMemcpyAsync(B.ck_theta[s], sp, sizeof(C) * V * nk, cudaMemcpyDeviceToDevice, st));
     }
-    const int hg = homog_at(step0 + i);
-    if (hg != up_homog) {
-      fa.homog = hg;
-      MEU_CUDA(cudaMemcpyAsync(B.dFwd, &fa, sizeof(fa), cudaMemcpyHostToDevice, st));
-      up_homog = hg;
+    const LanFusedArgs<R>* dArg = B.dFwd;
+    if (i >= last0) {
+      if (i == last0)
+        MEU_CUDA(cudaMemcpyAsync(B.dRec, B.hRec, sizeof(LanFusedArgs<R>) * (T - last0), cudaMemcpyHostToDevice, st));
+      dArg = B.dRec + (i - last0);
+    } else {
+      const int hg = homog_at(step0 + i);
+      if (hg != up_homog) {
+        fa.homog = hg;
+        MEU_CUDA(cudaMemcpyAsync(B.dFwd, &fa, sizeof(fa), cudaMemcpyHostToDevice, st));
+        up_homog = hg;
+      }
     }
-    if (!lan_fused_step<R>(N, V, sched, B.dFwd, 1, theta_ready ? LS_THETA_READY : 0, st, &prof, nb))
+    if (!lan_fused_step<R>(N, V, sched, dArg, 1, theta_ready ? LS_THETA_READY : 0, st, &prof, nb))
       throw CudaError("fused step not instantiated", MEU_ERR_UNSUPPORTED);
     theta_ready = true;
   }
+  // the handle ends at the final state
+  MEU_CUDA(cudaMemcpyAsync(phi, B.s_eta[T - last0], sizeof(R) * V * n3, cudaMemcpyDeviceToDevice, st));
+  MEU_CUDA(cudaMemcpyAsync(c, B.s_c[T - last0], sizeof(R) * n3, cudaMemcpyDeviceToDevice, st));
+  MEU_CUDA(cudaMemcpyAsync(keta, B.s_keta[T - last0], sizeof(C) * V * nk, cudaMemcpyDeviceToDevice, st));
+  MEU_CUDA(cudaMemcpyAsync(kc, B.s_kc[T - last0], sizeof(C) * nk, cudaMemcpyDeviceToDevice, st));
   step = step0 + T;
   // ---- loss and seed lam_T, nu_T (real) -> spectra
   KLAUNCH("adj_seed", (double)n3 * (2 * sizeof(R) + 16 + 2 * sizeof(R)),
           k_ad_seed<R><<<RED_BLOCKS, RED_THREADS, 0, st>>>(phi, c, dF, B.tgt_eta, B.tgt_c, B.lamT, B.nuT, n3, V, B.loss_part));
   MEU_CUDA(cudaMemsetAsync(B.acc, 0, sizeof(double) * 8, st));
+  MEU_CUDA(cudaMemsetAsync(B.partials, 0, sizeof(double) * ADJ_Q * PSTRIDE, st));
   {
     NbList l;
     for (int q = 0; q < Q_TOTAL; ++q) l.nb[q] = 0;
@@ -318,31 +353,20 @@ void Engine<R>::adjoint(int T, int K, const double* cons_tgt, const double* phi_
     auto c_p = [&](int j) { return j == 0 ? B.ck_c[seg] : B.s_c[j]; };
     auto keta_p = [&](int j) { return j == 0 ? B.ck_keta[seg] : B.s_keta[j]; };
     auto kc_p = [&](int j) { return j == 0 ? B.ck_kc[seg] : B.s_kc[j]; };
-    MEU_CUDA(cudaStreamSynchronize(st));  // hRec is about to be rewritten
-    for (int j = 0; j < S; ++j) {
-      LanFusedArgs<R> r = fa;
-      r.homog = homog_at(step0 + i0 + j);
-      r.eta = eta_p(j);
-      r.c = c_p(j);
-      r.Keta = keta_p(j);
-      r.Kc = kc_p(j);
-      r.eta_next = B.s_eta[j + 1];
-      r.c_next = B.s_c[j + 1];
-      r.Keta_out = B.s_keta[j + 1];
-      r.Kc_out = B.s_kc[j + 1];
-      r.rec_phi = B.s_phi[j];
-      r.rec_theta = B.s_theta[j];
-      B.hRec[j] = r;
+    if (seg < nck - 1) {
+      MEU_CUDA(cudaStreamSynchronize(st));  // hRec is about to be rewritten
+      for (int j = 0; j < S; ++j) B.hRec[j] = record(seg, j);
+      MEU_CUDA(cudaMemcpyAsync(B.dRec, B.hRec, sizeof(LanFusedArgs<R>) * S, cudaMemcpyHostToDevice, st));
+      // the segment starts from a checkpoint with the forward's theta^ (or, at the very first
+      // step, transforms theta itself as the forward did), so it repeats the forward exactly
+      const bool ck_theta = B.ck_has_theta[seg] != 0;
+      if (ck_theta)
+        MEU_CUDA(cudaMemcpyAsync(sp, B.ck_theta[seg], sizeof(C) * V * nk, cudaMemcpyDeviceToDevice, st));
+      for (int j = 0; j < S; ++j)
+        if (!lan_fused_step<R>(N, V, sched, B.dRec + j, 1, (j || ck_theta) ? LS_THETA_READY : 0, st, &prof, nb))
+          throw CudaError("fused step not instantiated", MEU_ERR_UNSUPPORTED);
     }
-    MEU_CUDA(cudaMemcpyAsync(B.dRec, B.hRec, sizeof(LanFusedArgs<R>) * S, cudaMemcpyHostToDevice, st));
-    // the segment starts from a checkpoint with the forward's theta^ (or, at the very first
-    // step, transforms theta itself as the forward did), so it repeats the forward exactly
-    const bool ck_theta = B.ck_has_theta[seg] != 0;
-    if (ck_theta) MEU_CUDA(cudaMemcpyAsync(sp, B.ck_theta[seg], sizeof(C) * V * nk, cudaMemcpyDeviceToDevice, st));
-    for (int j = 0; j < S; ++j)
-      if (!lan_fused_step<R>(N, V, sched, B.dRec + j, 1, (j || ck_theta) ? LS_THETA_READY : 0, st, &prof, nb))
-        throw CudaError("fused step not instantiated", MEU_ERR_UNSUPPORTED);
-    theta_ready = false;  // the engine's M now holds a recomputed step's theta^
+    theta_ready = false;  // the engine's M holds a recomputed step's theta^ or the seeds' transforms
     for (int m = S - 1; m >= 0; --m) {
       const int g = i0 + m;
       AdjArgs<R> a;
@@ -371,12 +395,13 @@ void Engine<R>::adjoint(int T, int K, const double* cons_tgt, const double* phi_
       a.twz = (const C*)fft->pz.tw;
       a.post = (const C*)fft->post_tw;
       a.err = d_err;
-      int nbq[Q_TOTAL];
-      if (!adj_step<R>(N, a, st, &prof, nbq)) throw CudaError("adjoint not instantiated", MEU_ERR_UNSUPPORTED);
-      NbList l;
-      for (int q = 0; q < Q_TOTAL; ++q) l.nb[q] = nbq[q];
-      KLAUNCH("adj_acc", 8.0 * (3 * nbq[AQ_X] + 2 * nbq[AQ_WG]), k_ad_acc<<<ADJ_Q, 256, 0, st>>>(B.partials, l, B.acc));
+      if (!adj_step<R>(N, a, st, &prof, nb)) throw CudaError("adjoint not instantiated", MEU_ERR_UNSUPPORTED);
     }
+  }
+  {
+    NbList l;
+    for (int q = 0; q < Q_TOTAL; ++q) l.nb[q] = nb[q];  // the same blocks in every step
+    KLAUNCH("adj_acc", 8.0 * (3 * nb[AQ_X] + 2 * nb[AQ_WG]), k_ad_acc<<<ADJ_Q, 256, 0, st>>>(B.partials, l, B.acc));
   }
   // ---- results
   double h[8];
