@@ -980,7 +980,13 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
   }
   el_ready = true;
   int total = 0;
+  struct FastPasses {  // the iterations' y and z passes on the rule's plans
+    FFT3& f;
+    explicit FastPasses(FFT3& g) : f(g) { f.fast = true; }
+    ~FastPasses() { f.fast = false; }
+  };
   if (!zeroth_only) {
+    FastPasses fast_passes(*fft);
     // The control runs on the device.  An iteration before the el_min_iter'th cannot end the
     // loop, so those are queued together: one wait of the host per step instead of one per
     // iteration where el_min_iter suffice.
