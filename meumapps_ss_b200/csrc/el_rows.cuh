@@ -469,7 +469,11 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
       for (int m = 0; m < 6; ++m) gam[m] = (double)e[2 * m];
       EnerVox o;
       ener_stress(E, K, gam, pv, VS, o, err);
-      double en = (1.0 - o.psum) * o.mat;
+      double en = (1.0 - o.psum) * o.mat, s2 = 0, cv = 0;
+      if (out.mode == 3) {
+        cv = K.c_mean[0] + (double)out.c[id];
+        each_variant(E.nvar, [&](int v) { s2 += (double)fv[v * VS] * (double)fv[v * VS]; });
+      }
       each_variant(E.nvar, [&](int v) {
         const double f = (double)fv[v * VS];
         double eg = 0;
@@ -481,7 +485,7 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
                            2.0 * (o.sig[3] * t[3] + o.sig[4] * t[4] + o.sig[5] * t[5]);
           const double pr = eta2 ? 2.0 * f : 30.0 * f * f * (f * f - 2.0 * f + 1.0);
           eg = pr * (o.mat - elp) - g * pr;
-        } else if (out.mode != 2) {
+        } else if (out.mode < 2) {
           return;
         }
         R* d = elg + v * n3 + id;
@@ -491,6 +495,11 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
           *d = (R)(f - out.dtl * (double)t + nz);
         } else if (out.mode == 0) {
           *d += (R)eg;
+        } else if (out.mode == 3) {
+          const meu_params& p = K.p;
+          const double e2 = f * f;
+          *d = (R)(p.lan_b * (p.lan_c2 - cv) * f - p.lan_c * e2 * f + p.lan_d * e2 * e2 * f +
+                   4.0 * p.cross_w * f * (s2 - e2) + eg);
         } else {
           *d = (R)eg;
         }

@@ -147,6 +147,12 @@ __global__ void __launch_bounds__(1024) k_el_zsum(const double* __restrict__ par
   for (int q = 0; q < 6; ++q) s[q] = __ldcg(out + q);
   el_control(A, s);
 }
+// fixed-order sum of n values into *out
+__global__ void __launch_bounds__(1024) k_sum(const double* __restrict__ p, int64_t n, double* out) {
+  double acc = 0;
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) acc += p[i];
+  block_reduce_store(acc, 0, out);
+}
 __global__ void k_el_control(const double* sums, const __grid_constant__ ElCtlArgs A) {
   if (threadIdx.x == 0) el_control(A, sums);
 }
@@ -409,6 +415,8 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
       }
       el_gen.nvar = V;
       el_gen.numph = p.numph;
+      if (p.model == MEU_MODEL_LANDAU && axis_ok(p.nz))
+        zdiv_part = dalloc<double>((int64_t)V * z_div_blocks<R>(p.ny * hK.nxh));
       for (int n = 1; n < p.numph; ++n) {
         el_gen.lo[n] = hK.ph_lo[n + 1];
         el_gen.hi[n] = hK.ph_hi[n + 1];
@@ -1065,6 +1073,21 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
                 dK, ph_for_ppr, pphi, strain, el_en, elg, eo.mode, eta2, partials, d_err));
 }
 
+template <typename R>
+ZDivArgs<R> Engine<R>::zdiv_args() const {
+  ZDivArgs<R> Z{};
+  Z.sp = spec(0);
+  Z.stride = nk;
+  Z.inner = P.ny * hK.nxh;
+  Z.nxh = hK.nxh;
+  Z.nx = P.nx;
+  Z.ny = P.ny;
+  Z.scale = 1.0 / ((double)P.nx * P.ny * P.nz);
+  Z.wx = 6.283185307179586476925286766559 / (double)P.nx;
+  Z.wy = 6.283185307179586476925286766559 / (double)P.ny;
+  return Z;
+}
+
 // ------------------------------------------------------------------- KKS step
 template <typename R>
 void Engine<R>::kks_step(meu_diag* d) {
@@ -1130,7 +1153,7 @@ void Engine<R>::kks_step(meu_diag* d) {
   bool rhs_done = false;
   if (step >= P.elastep0 && P.elastic != MEU_ELAST_NONE) {
     rhs_done = el_fused_rows;
-    elastic(phi, fd, EnerOut<R>{rhs_done ? 2 : 0, P.dt * P.b_mob, P.dt, noise_live ? noise : nullptr}, false);
+    elastic(phi, fd, EnerOut<R>{rhs_done ? 2 : 0, P.dt * P.b_mob, P.dt, noise_live ? noise : nullptr, nullptr}, false);
   } else {
     MEU_CUDA(cudaMemsetAsync(el_en, 0, sizeof(R) * n3, st));
   }
@@ -1151,16 +1174,7 @@ void Engine<R>::kks_step(meu_diag* d) {
     R* wp = rhs_done ? fd : field(wr, E);
     if (!rhs_done)
       KLAUNCH("tdgl_pre", 4.0 * V * n3 * sizeof(R), k_tdgl_pre<R><<<grid_for((int64_t)V * n3, 256), 256, 0, st>>>(phi, fd, noise, wp, (int64_t)V * n3, P.dt * P.b_mob, P.dt));
-    ZDivArgs<R> Z{};
-    Z.sp = spec(0);
-    Z.stride = nk;
-    Z.inner = P.ny * hK.nxh;
-    Z.nxh = hK.nxh;
-    Z.nx = P.nx;
-    Z.ny = P.ny;
-    Z.scale = 1.0 / ((double)P.nx * P.ny * P.nz);
-    Z.wx = 6.283185307179586476925286766559 / (double)P.nx;
-    Z.wy = 6.283185307179586476925286766559 / (double)P.ny;
+    ZDivArgs<R> Z = zdiv_args();
     PtrList<const R> in{};
     PtrList<R> out{};
     for (int e = 0; e < E; ++e) {
@@ -1355,15 +1369,22 @@ void Engine<R>::landau_step(meu_diag* d) {
   const bool het = elast && P.elastic == MEU_ELAST_HETERO;
   R* mu = field(wr, 0);
   KLAUNCH("lan_a", (double)(2 * V + 2) * n3 * sizeof(R), k_lan_a<R><<<RED_BLOCKS, RED_THREADS, 0, st>>>(dK, c, phi, pphi, mu, partials));
-  {
+  // only homogeneous elasticity needs theta^ here: otherwise mu is transformed alone
+  PtrList<C> S1 = specs(0, V + 1);
+  if (homog) {
     std::vector<const R*> in;
     for (int v = 0; v < V; ++v) in.push_back(field(pphi, v));
     in.push_back(mu);
     fwd_list(in, 0);
+  } else {
+    fwd({mu}, 0);
+    S1.p[V] = spec(0);
   }
-  KLAUNCH("lan_k1", (double)(homog ? 3 * V + 4 : 2 * V + 4) * nk * sizeof(C),
-          k_lan_k1<R><<<g_lan_k1, RED_THREADS, 0, st>>>(dK, specs(0, V + 1), V, kc, keta, homog ? 1 : 0,
-                                                          P.diag_energy, partials, d_err));
+  // on the row path the update of eta^ sums its gradient energy
+  const bool zstate = zdiv_part != nullptr;
+  KLAUNCH("lan_k1", (double)(homog ? 3 * V + 4 : (zstate ? 0 : V) + 4) * nk * sizeof(C),
+          k_lan_k1<R><<<g_lan_k1, RED_THREADS, 0, st>>>(dK, S1, V, kc, keta, homog ? 1 : 0, P.diag_energy, zstate ? 0 : 1,
+                                                          partials, d_err));
   R* phel = field(wr, 1);  // V fields: strain interaction (homog) or el_grad (hetero)
   {
     std::vector<R*> out;
@@ -1372,20 +1393,48 @@ void Engine<R>::landau_step(meu_diag* d) {
       out.push_back(c2);
       inv_list(0, out);
     } else {
-      inv_list(V, {c2});
+      inv_list(0, {c2});
     }
   }
   last_iters = 0;
-  if (het) {
-    // P_phi = theta (already in pphi), elener gives el_grad into phel
-    elastic(phi, phel, EnerOut<R>{1, 0.0, 0.0, nullptr}, false);
-  } else if (!homog) {
-    MEU_CUDA(cudaMemsetAsync(el_en, 0, sizeof(R) * n3, st));
+  R* rhs = pphi;  // the TDGL driving force
+  if (het && el_fused_rows) {
+    // elener adds its el_grad to the local force
+    elastic(phi, phel, EnerOut<R>{3, 0.0, 0.0, nullptr, c}, false);
+    rhs = phel;
+  } else {
+    if (het) {
+      // P_phi = theta (already in pphi), elener gives el_grad into phel
+      elastic(phi, phel, EnerOut<R>{1, 0.0, 0.0, nullptr, nullptr}, false);
+    } else if (!homog) {
+      MEU_CUDA(cudaMemsetAsync(el_en, 0, sizeof(R) * n3, st));
+    }
+    KLAUNCH("lan_b", (double)(3 * V + 1) * n3 * sizeof(R), k_lan_b<R><<<gridr(), 256, 0, st>>>(dK, c, phi, elast ? phel : nullptr, homog ? 1 : 0, pphi));
   }
-  KLAUNCH("lan_b", (double)(3 * V + 1) * n3 * sizeof(R), k_lan_b<R><<<gridr(), 256, 0, st>>>(dK, c, phi, elast ? phel : nullptr, homog ? 1 : 0, pphi));
-  {
+  if (zstate) {
+    ZDivArgs<R> Z = zdiv_args();
+    Z.state = keta;
+    Z.part = P.diag_energy ? zdiv_part : nullptr;
+    PtrList<const R> in{};
+    PtrList<R> out{};
+    for (int v = 0; v < V; ++v) {
+      in.p[v] = rhs + (int64_t)v * n3;
+      out.p[v] = field(phi, v);
+      Z.s[v] = P.dt * P.b_mob;
+      for (int i = 0; i < 9; ++i) Z.g[v][i] = P.grad_coeff[v][i];
+    }
+    const PtrList<C> S = specs(0, V);
+    fft->forward_x<R>(in, S, V, st);
+    fft->pass_y<R>(S, V, true, st);
+    KLAUNCH("tdgl", 4.0 * V * nk * sizeof(C), z_div_launch<R>(Z, V, *fft, st));
+    if (Z.part)
+      KLAUNCH("finalize", 8.0 * V * z_div_blocks<R>(Z.inner),
+              k_sum<<<1, 1024, 0, st>>>(zdiv_part, (int64_t)V * z_div_blocks<R>(Z.inner), partials + (int64_t)Q_FINT2 * PSTRIDE));
+    fft->pass_y<R>(S, V, false, st);
+    fft->inverse_x<R>(S, out, V, st);
+  } else {
     std::vector<const R*> in;
-    for (int v = 0; v < V; ++v) in.push_back(field(pphi, v));
+    for (int v = 0; v < V; ++v) in.push_back(field(rhs, v));
     fwd_list(in, 0);
     KLAUNCH("tdgl", 4.0 * V * nk * sizeof(C), k_tdgl_state<R><<<gridk(), 256, 0, st>>>(dK, specs(0, V), V, keta, P.dt * P.b_mob));
     std::vector<R*> out;

@@ -101,20 +101,26 @@ void axis_launch(int axis, const AxisArgs<R>& A, int nf, const FFT3& f, const vo
 template <typename R>
 struct ZDivArgs {
   cplx<R>* sp;
+  cplx<R>* state;  // NULL, or the spectral state (same stride)
+  double* part;    // NULL, or [nf][z_div_blocks] partials of the state's gradient energy
   int64_t stride;
   int inner, nxh, nx, ny;
   double scale, wx, wy;
   double s[MEU_MAX_VAR + MEU_MAX_EL], g[MEU_MAX_VAR + MEU_MAX_EL][9];
 };
 template <typename R>
+constexpr int z_div_blocks(int inner) { return (inner + 128 / (2 * (int)sizeof(R)) - 1) / (128 / (2 * (int)sizeof(R))); }
+template <typename R>
 void z_div_launch(const ZDivArgs<R>& A, int nf, const FFT3& f, cudaStream_t st);
 // what elener does with the driving force eg: 0 elg += eg; 1 elg = eg; 2 the right-hand side of
-// the TDGL update, elg = phi - dtl (elg + eg) + dt noise (Multi_MEUMAPPS.f:957-987)
+// the TDGL update, elg = phi - dtl (elg + eg) + dt noise (Multi_MEUMAPPS.f:957-987); 3 the Landau
+// driving force, elg = df/deta + eg (constants and mean concentration from DevConst)
 template <typename R>
 struct EnerOut {
   int mode;
   double dtl, dt;
   const R* noise;  // NULL: zero
+  const R* c;      // mode 3: the concentration
 };
 // x-direction work of one elastic iteration in one pass, and elener on the same row spectra
 // (el_rows.cuh): sp the six row spectra, nk apart; tw: exp(-2 pi i n / nx), n < nx
@@ -424,6 +430,8 @@ class Engine : public EngineBase {
   // by up to 2e-3, so these decks keep the separate passes on their own radix plans.
   bool keep_rounding = false;
   KksPar kks_par{};
+  double* zdiv_part = nullptr;        // Landau on the row path: partials of z_div's gradient energy
+  ZDivArgs<R> zdiv_args() const;      // sp = spec(0), grid constants
   bool noise_live = false;            // phi_noise may be nonzero
   bool el_state = false;              // heterogeneous elasticity keeps a state between steps
   C* es = nullptr;

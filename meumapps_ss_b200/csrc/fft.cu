@@ -305,6 +305,23 @@ static bool cols_s(bool mix, int L, int pv, int ct, int nf, int outer, int inner
   return dispatch_len(L, pv, go) || (mix && cols_mix<R, FWD>(L, nf, outer, inner, ostride, in, out, tw, scale, st));
 }
 
+// Radix plan and column-tile factor of the power-of-two passes on the default plan (pv 0, ct 1), by
+// length, direction and precision, where by_rule() lets it choose.  The forward pass loads its
+// first butterflies from global memory and stores through the digit reversal, the inverse the
+// other way round, and radix 16 needs twice the registers in FP64, so they do not agree.  us per
+// launch of six fields, (0, 1) / chosen: FP32 256^3 y 163 / 139 forward, 173 / 126 inverse; FP32
+// 128^3 y inverse 22.7 / 20.5; FP64 128^3 y inverse 40.7 / 34.5 (forward 40.8, radix 16 50.5); FP64
+// 256^3 y inverse 287 / 226; FP64 512 columns 339 / 331 forward.
+struct LinePick {
+  int pv, ct;
+};
+static LinePick pick_cols(bool fp64, int L, bool fwd) {
+  if (!fp64) return L == 256 || (L == 128 && !fwd) ? LinePick{2, 1} : LinePick{0, 1};
+  if (!fwd && L == 128) return {2, 1};
+  if (!fwd && L == 256) return {2, 2};
+  return {0, L == 512 ? 2 : 1};
+}
+
 static inline int col_tile(int L, bool fp64) {
   if (fp64) return L >= 256 ? 8 : 16;
   return 16;
@@ -355,14 +372,15 @@ void FFT3::pass_y(const PtrList<cplx<R>>& in, const PtrList<cplx<R>>& out, int n
   const int tm = col_tile(ny, sizeof(R) == 8);
   const size_t s2 = (size_t)ny * tm * sizeof(C);
   const dim3 g2((unsigned)(nz * ((nxh + tm - 1) / tm)), nf);
+  const LinePick pk = by_rule(sizeof(R) == 8) ? pick_cols(sizeof(R) == 8, ny, fwd) : LinePick{pv, ct};
   HookScope hs_(hook, fwd ? "fft_y_fwd" : "fft_y_inv", 2.0 * nf * nk() * sizeof(C), st);
   if (fwd) {
-    if (!cols_s<R, true>(mix, ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, in, out, py.tw, (R)1, st)) {
+    if (!cols_s<R, true>(mix, ny, pk.pv, pk.ct, nf, nz, nxh, (int64_t)ny * nxh, in, out, py.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, true>, s2);
       k_cols<R, true><<<g2, 256, s2, st>>>(in, out, nxh, (int64_t)ny * nxh, tm, py, (R)1);
     }
   } else {
-    if (!cols_s<R, false>(mix, ny, pv, ct, nf, nz, nxh, (int64_t)ny * nxh, in, out, py.tw, (R)1, st)) {
+    if (!cols_s<R, false>(mix, ny, pk.pv, pk.ct, nf, nz, nxh, (int64_t)ny * nxh, in, out, py.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, false>, s2);
       k_cols<R, false><<<g2, 256, s2, st>>>(in, out, nxh, (int64_t)ny * nxh, tm, py, (R)1);
     }
@@ -378,15 +396,16 @@ void FFT3::pass_z(const PtrList<cplx<R>>& buf, int nf, bool fwd, cudaStream_t st
   const size_t s3 = (size_t)nz * tm * sizeof(C);
   const int inner = ny * nxh;
   const dim3 g3((unsigned)((inner + tm - 1) / tm), nf);
+  const LinePick pk = by_rule(sizeof(R) == 8) ? pick_cols(sizeof(R) == 8, nz, fwd) : LinePick{pv, ct};
   HookScope hs_(hook, fwd ? "fft_z_fwd" : "fft_z_inv", 2.0 * nf * nk() * sizeof(C), st);
   if (fwd) {
     const R scale = (R)(1.0 / ((double)nx * ny * nz));
-    if (!cols_s<R, true>(mix, nz, pv, ct, nf, 1, inner, 0, buf, buf, pz.tw, scale, st)) {
+    if (!cols_s<R, true>(mix, nz, pk.pv, pk.ct, nf, 1, inner, 0, buf, buf, pz.tw, scale, st)) {
       set_smem<R>((const void*)k_cols<R, true>, s3);
       k_cols<R, true><<<g3, 256, s3, st>>>(buf, buf, inner, 0, tm, pz, scale);
     }
   } else {
-    if (!cols_s<R, false>(mix, nz, pv, ct, nf, 1, inner, 0, buf, buf, pz.tw, (R)1, st)) {
+    if (!cols_s<R, false>(mix, nz, pk.pv, pk.ct, nf, 1, inner, 0, buf, buf, pz.tw, (R)1, st)) {
       set_smem<R>((const void*)k_cols<R, false>, s3);
       k_cols<R, false><<<g3, 256, s3, st>>>(buf, buf, inner, 0, tm, pz, (R)1);
     }

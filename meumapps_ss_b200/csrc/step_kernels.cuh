@@ -811,11 +811,11 @@ __global__ void __launch_bounds__(RED_THREADS) k_lan_a(const DevConst* __restric
 // energy, and the Cahn-Hilliard update of the spectral state
 //   dc^ <- (dc^ - dt M k^2 mu^) / (1 + dt M kappa_c k^4),  dc^(0) = 0.
 // sp: [theta_0..V-1, mu] on entry; [phi_0..V-1 (homog), dc_new] on exit.
-// kc: dc^ state (read, updated); keta: eta^ state (read for the energy).
+// kc: dc^ state (read, updated); keta: eta^ state (read for the energy, unless its update sums it).
 template <typename R>
 __global__ void __launch_bounds__(RED_THREADS) k_lan_k1(const DevConst* __restrict__ Kp, PtrList<cplx<R>> sp, int V,
                                                         cplx<R>* __restrict__ kc, const cplx<R>* __restrict__ keta,
-                                                        int homog, int energy, double* partials, int* err) {
+                                                        int homog, int energy, int eta_energy, double* partials, int* err) {
   const DevConst& K = *Kp;
   const meu_params& p = K.p;
   const int64_t nk = K.nk;
@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_lan_k1(const DevConst* __restri
     if (energy) {
       const double bb = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
       double f = p.kappa_c * bb * (cr * cr + ci * ci);
-      for (int v = 0; v < V; ++v) {
+      for (int v = 0; v < (eta_energy ? V : 0); ++v) {
         double er, ei;
         ld2(keta[(int64_t)v * nk + id], er, ei);
         f += kkappak_b(p.grad_coeff[v], b) * (er * er + ei * ei);
