@@ -444,7 +444,7 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
   MEU_CUDA(cudaMemset(el_ticket, 0, sizeof(unsigned)));
   MEU_CUDA(cudaHostAlloc((void**)&h_ctl, sizeof(ElCtl), cudaHostAllocDefault));
   dK = dalloc<DevConst>(1);
-  MEU_CUDA(cudaHostAlloc((void**)&h_results, sizeof(double) * Q_TOTAL, cudaHostAllocDefault));
+  MEU_CUDA(cudaHostAlloc((void**)&h_results, sizeof(double) * (Q_TOTAL + PIN_ROWS * Q_STEP_COUNT), cudaHostAllocDefault));
   MEU_CUDA(cudaHostAlloc((void**)&h_err, sizeof(int), cudaHostAllocDefault));
   int ops[Q_TOTAL];
   for (int q = 0; q < Q_TOTAL; ++q) ops[q] = 0;
@@ -926,8 +926,9 @@ void Engine<R>::run_noise(int nsteps, meu_ran2_state* rng, double sd, meu_diag* 
       }
       kks_step(nullptr);
     }
-    check_err();
-    flush_hist(diag ? diag + done : nullptr);
+    queue_flush(st);
+    MEU_CUDA(cudaStreamSynchronize(st));
+    finish_flush(diag ? diag + done : nullptr);
     done += chunk;
   }
 }
@@ -1462,13 +1463,18 @@ void Engine<R>::end_step(meu_diag* d, int clip) {
 template <typename R>
 void Engine<R>::flush_hist(meu_diag* diag) {
   if (hist_n == 0) return;
-  std::vector<double> h((size_t)hist_n * Q_STEP_COUNT);
-  MEU_CUDA(cudaMemcpyAsync(h.data(), hist, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
-  MEU_CUDA(cudaStreamSynchronize(st));
+  std::vector<double> h;
+  if (!hist_pinned) {
+    h.resize((size_t)hist_n * Q_STEP_COUNT);
+    MEU_CUDA(cudaMemcpyAsync(h.data(), hist, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
+    MEU_CUDA(cudaStreamSynchronize(st));
+  }
+  const double* rows = hist_pinned ? h_results + Q_TOTAL : h.data();
+  hist_pinned = false;
   const double sn3 = (double)n3;
   const bool lan = P.model == MEU_MODEL_LANDAU;
   for (int i = 0; i < hist_n; ++i) {
-    const double* r = h.data() + (size_t)i * Q_STEP_COUNT;
+    const double* r = rows + (size_t)i * Q_STEP_COUNT;
     if (diag) {
       meu_diag* d = diag + i;
       d->step = hist_step[i];
@@ -1502,6 +1508,22 @@ void Engine<R>::flush_hist(meu_diag* diag) {
   hist_n = 0;
 }
 
+// The end of a call's chunk: the error word and the history rows come back together behind the
+// steps, so a call waits once (a 32^3 step of 20 us paid two waits and a pageable copy).
+template <typename R>
+void Engine<R>::queue_flush(cudaStream_t s) {
+  MEU_CUDA(cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+  hist_pinned = hist_n > 0 && hist_n <= PIN_ROWS;
+  if (hist_pinned)
+    MEU_CUDA(cudaMemcpyAsync(h_results + Q_TOTAL, hist, sizeof(double) * (size_t)hist_n * Q_STEP_COUNT,
+                             cudaMemcpyDeviceToHost, s));
+}
+template <typename R>
+void Engine<R>::finish_flush(meu_diag* diag) {
+  if (*h_err) raise_err(*h_err);
+  flush_hist(diag);
+}
+
 template <typename R>
 void Engine<R>::run(int nsteps, meu_diag* diag) {
   int done = 0;
@@ -1517,8 +1539,9 @@ void Engine<R>::run(int nsteps, meu_diag* diag) {
         else landau_step(nullptr);
       }
     }
-    check_err();
-    flush_hist(diag ? diag + done : nullptr);
+    queue_flush(st);
+    MEU_CUDA(cudaStreamSynchronize(st));
+    finish_flush(diag ? diag + done : nullptr);
     done += chunk;
   }
 }

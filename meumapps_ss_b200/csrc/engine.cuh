@@ -382,6 +382,8 @@ class Engine : public EngineBase {
     return l;
   }
   void check_err();
+  void queue_flush(cudaStream_t s);     // error word and history rows to pinned memory (no wait)
+  void finish_flush(meu_diag* diag);    // after s has been waited for: check_err and flush_hist
   void raise_err(int code);  // clears the device's error word and throws
   void finalize(int q0, int nq, double* out = nullptr, const int* nbs = nullptr);
   void elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& out, bool zeroth_only);
@@ -463,6 +465,9 @@ class Engine : public EngineBase {
   void flush_hist(meu_diag* diag);
   static constexpr int HIST_MAX = 4096;
   double* hist = nullptr;  // per-step reductions [HIST_MAX][Q_STEP_COUNT]
+  // rows that fit the pinned copy behind h_results (a longer call copies its own)
+  static constexpr int PIN_ROWS = 128;
+  bool hist_pinned = false;  // the pinned copy holds rows 0 .. hist_n - 1
   double* cmean_acc = nullptr;
   int hist_n = 0;
   std::vector<int64_t> hist_step = std::vector<int64_t>(HIST_MAX);

@@ -364,12 +364,13 @@ void EnsembleT<R>::run(int nsteps, meu_diag* diag) {
       }
       i += k;
     }
+    // every member's error word and history behind the last step, one wait for all of them
+    for (auto& e : mem) e->queue_flush(st);
     MEU_CUDA(cudaStreamSynchronize(st));
     for (int m = 0; m < members; ++m) {
       Engine<R>& e = *mem[m];
       e.step = step;
-      e.check_err();
-      e.flush_hist(diag ? diag + (int64_t)m * nsteps + done : nullptr);
+      e.finish_flush(diag ? diag + (int64_t)m * nsteps + done : nullptr);
     }
     done += chunk;
   }
