@@ -85,27 +85,27 @@ void adj_step_n(const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb)
 }
 
 // one adjoint step of V >= 2 variants (adjoint.cuh: EA_v, B1_v, B2_v, B3_v, C_v, D_v)
-template <typename R, int N, int V>
+template <typename R, int N, int V, int PV>
 void adj_step_nv(const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb) {
   using C = cplx<R>;
-  using P = fz::Plane<R, N, adj::NTP, adj::PV>;
+  using P = fz::Plane<R, N, adj::NTP, PV>;
   constexpr int TM = lf::col_tile_default<R>(), NXH = N / 2 + 1, tiles = N * NXH / TM;
   const double n3 = (double)N * N * N, nk = (double)N * N * NXH;
   const size_t sc = sizeof(C) * ((size_t)N * V * TM + N * Tw<C>::K);
   const size_t sp = P::smem_bytes();
-  lf::ensure_smem(adj::k_ad_ea_v<R, N, V>, sc);
-  lf::ensure_smem(adj::k_ad_c_v<R, N, V>, sc);
-  lf::ensure_smem(adj::k_ad_b1_v<R, N>, sp);
-  lf::ensure_smem(adj::k_ad_b3_v<R, N>, sp);
-  lf::ensure_smem(adj::k_ad_d_v<R, N>, sp);
+  lf::ensure_smem(adj::k_ad_ea_v<R, N, V, PV>, sc);
+  lf::ensure_smem(adj::k_ad_c_v<R, N, V, PV>, sc);
+  lf::ensure_smem(adj::k_ad_b1_v<R, N, PV>, sp);
+  lf::ensure_smem(adj::k_ad_b3_v<R, N, PV>, sp);
+  lf::ensure_smem(adj::k_ad_d_v<R, N, PV>, sp);
   {
     lf::Scope s(hook, "adj_z_lambda", (3.0 + 2.0) * V * nk * sizeof(C) + 2.0 * nk * sizeof(C), st);
-    adj::k_ad_ea_v<R, N, V><<<tiles, lf::NT, sc, st>>>(a);
+    adj::k_ad_ea_v<R, N, V, PV><<<tiles, lf::NT, sc, st>>>(a);
     MEU_CHECK_LAUNCH();
   }
   {
     lf::Scope s(hook, "adj_plane_w", V * (nk * sizeof(C) + n3 * sizeof(R)), st);
-    adj::k_ad_b1_v<R, N><<<dim3(N, V), adj::NTP, sp, st>>>(a);
+    adj::k_ad_b1_v<R, N, PV><<<dim3(N, V), adj::NTP, sp, st>>>(a);
     MEU_CHECK_LAUNCH();
   }
   {
@@ -115,17 +115,17 @@ void adj_step_nv(const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb
   }
   {
     lf::Scope s(hook, "adj_plane_h", V * (nk * sizeof(C) + n3 * sizeof(R)), st);
-    adj::k_ad_b3_v<R, N><<<dim3(N, V), adj::NTP, sp, st>>>(a);
+    adj::k_ad_b3_v<R, N, PV><<<dim3(N, V), adj::NTP, sp, st>>>(a);
     MEU_CHECK_LAUNCH();
   }
   {
     lf::Scope s(hook, "adj_z_nu", 2.0 * V * nk * sizeof(C) + 2.0 * nk * sizeof(C), st);
-    adj::k_ad_c_v<R, N, V><<<tiles, lf::NT, sc, st>>>(a);
+    adj::k_ad_c_v<R, N, V, PV><<<tiles, lf::NT, sc, st>>>(a);
     MEU_CHECK_LAUNCH();
   }
   {
     lf::Scope s(hook, "adj_plane_lambda", V * ((a.lam_out ? 1.0 : 2.0) * nk * sizeof(C) + 3.0 * n3 * sizeof(R)), st);
-    adj::k_ad_d_v<R, N><<<dim3(N, V), adj::NTP, sp, st>>>(a);
+    adj::k_ad_d_v<R, N, PV><<<dim3(N, V), adj::NTP, sp, st>>>(a);
     MEU_CHECK_LAUNCH();
   }
   for (int q = 0; q < Q_TOTAL; ++q) nb[q] = 0;
@@ -133,13 +133,26 @@ void adj_step_nv(const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb
   nb[AQ_WG] = nb[AQ_EA] = RED_BLOCKS;
 }
 
+// the radix plan fixes the order of the spectra: plan 0, and plan 2 where it is the default
+template <typename R, int N, int V>
+void adj_step_pv(int pv, const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb) {
+  if constexpr (N == 128) {
+    if (pv == 2) return adj_step_nv<R, N, V, 2>(a, st, hook, nb);
+  }
+  if (pv != 0) throw CudaError("the adjoint has no kernels of this radix plan", MEU_ERR_UNSUPPORTED);
+  adj_step_nv<R, N, V, 0>(a, st, hook, nb);
+}
+
 template <typename R, int N>
-void adj_step_any(const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb) {
+void adj_step_any(int pv, const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb) {
   switch (a.V) {
-    case 1: adj_step_n<R, N>(a, st, hook, nb); break;
-    case 2: adj_step_nv<R, N, 2>(a, st, hook, nb); break;
-    case 3: adj_step_nv<R, N, 3>(a, st, hook, nb); break;
-    case 4: adj_step_nv<R, N, 4>(a, st, hook, nb); break;
+    case 1:
+      if (pv != 0) throw CudaError("the adjoint has no kernels of this radix plan", MEU_ERR_UNSUPPORTED);
+      adj_step_n<R, N>(a, st, hook, nb);
+      break;
+    case 2: adj_step_pv<R, N, 2>(pv, a, st, hook, nb); break;
+    case 3: adj_step_pv<R, N, 3>(pv, a, st, hook, nb); break;
+    case 4: adj_step_pv<R, N, 4>(pv, a, st, hook, nb); break;
     default: throw CudaError("adjoint: 1 to 4 variants", MEU_ERR_UNSUPPORTED);
   }
 }
@@ -147,13 +160,13 @@ void adj_step_any(const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* n
 }  // namespace
 
 template <typename R>
-bool adj_step(int N, const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb) {
+bool adj_step(int N, int pv, const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb) {
   switch (N) {
-    case 32: adj_step_any<R, 32>(a, st, hook, nb); return true;
-    case 48: adj_step_any<R, 48>(a, st, hook, nb); return true;
-    case 64: adj_step_any<R, 64>(a, st, hook, nb); return true;
-    case 96: adj_step_any<R, 96>(a, st, hook, nb); return true;
-    case 128: adj_step_any<R, 128>(a, st, hook, nb); return true;
+    case 32: adj_step_any<R, 32>(pv, a, st, hook, nb); return true;
+    case 48: adj_step_any<R, 48>(pv, a, st, hook, nb); return true;
+    case 64: adj_step_any<R, 64>(pv, a, st, hook, nb); return true;
+    case 96: adj_step_any<R, 96>(pv, a, st, hook, nb); return true;
+    case 128: adj_step_any<R, 128>(pv, a, st, hook, nb); return true;
     default: return false;
   }
 }
@@ -197,7 +210,9 @@ void Engine<R>::adjoint(int T, int K, const double* cons_tgt, const double* phi_
   if (!fused || V < 1 || V > 4)
     throw CudaError("the adjoint covers the fused Landau step with 1 to 4 order parameters", MEU_ERR_UNSUPPORTED);
   const int tm_def = sizeof(R) == 4 ? 16 : 8;
-  if (sched.pv != 0 || sched.ntp != 512 || (sched.tm != 0 && sched.tm != tm_def))
+  const LanSched def = lan_default(P.nx, V, sizeof(R) == 8);
+  const bool is_def = sched.pv == def.pv && sched.ntp == def.ntp && sched.tm == def.tm;
+  if (!is_def && (sched.pv != 0 || sched.ntp != 512 || sched.tm != tm_def))
     throw CudaError("the adjoint runs on the default schedule", MEU_ERR_UNSUPPORTED);
   if (T < 1 || K < 1 || !cons_tgt || !phi_tgt) throw CudaError("adjoint: bad arguments", MEU_ERR_BADARG);
   if (!fields_set) throw CudaError("adjoint: set the initial fields first", MEU_ERR_BADARG);
@@ -395,7 +410,7 @@ void Engine<R>::adjoint(int T, int K, const double* cons_tgt, const double* phi_
       a.twz = (const C*)fft->pz.tw;
       a.post = (const C*)fft->post_tw;
       a.err = d_err;
-      if (!adj_step<R>(N, a, st, &prof, nb)) throw CudaError("adjoint not instantiated", MEU_ERR_UNSUPPORTED);
+      if (!adj_step<R>(N, sched.pv, a, st, &prof, nb)) throw CudaError("adjoint not instantiated", MEU_ERR_UNSUPPORTED);
     }
   }
   {
@@ -436,8 +451,8 @@ void Engine<R>::adjoint(int T, int K, const double* cons_tgt, const double* phi_
   }
 }
 
-template bool adj_step<float>(int, const AdjArgs<float>&, cudaStream_t, LaunchHook*, int*);
-template bool adj_step<double>(int, const AdjArgs<double>&, cudaStream_t, LaunchHook*, int*);
+template bool adj_step<float>(int, int, const AdjArgs<float>&, cudaStream_t, LaunchHook*, int*);
+template bool adj_step<double>(int, int, const AdjArgs<double>&, cudaStream_t, LaunchHook*, int*);
 template void Engine<float>::adjoint(int, int, const double*, const double*, double*, double*, double*);
 template void Engine<double>::adjoint(int, int, const double*, const double*, double*, double*, double*);
 template void adj_buffers_free<float>(AdjBuffers<float>*);

@@ -80,6 +80,6 @@ enum AdjQ : int { AQ_X = 0, AQ_Y, AQ_Z, AQ_WG, AQ_EA, ADJ_Q };
 
 // launches of one adjoint step and of the loss seed (adjoint.cu)
 template <typename R>
-bool adj_step(int N, const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb);
+bool adj_step(int N, int pv, const AdjArgs<R>& a, cudaStream_t st, LaunchHook* hook, int* nb);
 
 }  // namespace meu

@@ -16,7 +16,7 @@ __device__ __forceinline__ void block_reduce_add(double v, double* out) {
 
 using lf::NT;
 constexpr int NTP = 512;
-constexpr int PV = 0;
+constexpr int PV = 0;  // the radix plan of the one-variant kernels; the others take the handle's
 
 // g(k) = -(sig0 b)^T Omega (sig0 b) for one variant (same Q as the forward Green operator)
 __device__ __forceinline__ double green_scalar(const LanFusedConst& F, const double av[3], const double b[3]) {
@@ -270,7 +270,7 @@ __device__ __forceinline__ void sig_b(const double* sg, const double b[3], doubl
 }
 
 // EA_v: z FFT of lam_{v,n+1} -> w^_v = H_v lam^_v (+ X, Y, Z sums) -> z iFFT, V fields
-template <typename R, int N, int V>
+template <typename R, int N, int V, int PV>
 __global__ void __launch_bounds__(NT) k_ad_ea_v(AdjArgs<R> a) {
   using C = cplx<R>;
   constexpr int TM = lf::col_tile_default<R>(), NXH = N / 2 + 1, LN = V * TM;
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(NT) k_ad_ea_v(AdjArgs<R> a) {
 }
 
 // B1_v: plane (z, v): xy iFFT of w^_v -> real w_v
-template <typename R, int N>
+template <typename R, int N, int PV>
 __global__ void __launch_bounds__(NTP) k_ad_b1_v(AdjArgs<R> a) {
   using P = fz::Plane<R, N, NTP, PV>;
   using C = cplx<R>;
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_ad_b2_v(AdjArgs<R> a, int64_t n
 }
 
 // B3_v: plane (z, v): xy FFT of the real h_v -> M-form field v
-template <typename R, int N>
+template <typename R, int N, int PV>
 __global__ void __launch_bounds__(NTP) k_ad_b3_v(AdjArgs<R> a) {
   using P = fz::Plane<R, N, NTP, PV>;
   using C = cplx<R>;
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(NTP) k_ad_b3_v(AdjArgs<R> a) {
 }
 
 // C_v: z FFT of h^_v -> nu^ update (B sum_v h^_v), r^_q -> z iFFT, V fields
-template <typename R, int N, int V>
+template <typename R, int N, int V, int PV>
 __global__ void __launch_bounds__(NT) k_ad_c_v(AdjArgs<R> a) {
   using C = cplx<R>;
   constexpr int TM = lf::col_tile_default<R>(), NXH = N / 2 + 1, LN = V * TM;
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(NT) k_ad_c_v(AdjArgs<R> a) {
 }
 
 // D_v: plane (z, q): xy iFFT of r_q -> lam_q = a_q + 2 eta_q r_q -> xy FFT (or lam_0 out)
-template <typename R, int N>
+template <typename R, int N, int PV>
 __global__ void __launch_bounds__(NTP) k_ad_d_v(AdjArgs<R> a) {
   using P = fz::Plane<R, N, NTP, PV>;
   using C = cplx<R>;

@@ -461,6 +461,7 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
     MEU_CUDA(cudaMemset(kc, 0, sizeof(C) * nk));
   }
   fused = lan_fused_supported(p) && !(p.flags & MEU_FLAG_GENERIC);
+  if (fused) sched = lan_default(p.nx, V, sizeof(R) == 8);
   if (fused) {
     LanFusedConst F;
     memset(&F, 0, sizeof(F));

@@ -295,7 +295,7 @@ class Engine : public EngineBase {
     }
     out3[0] = sched.pv;
     out3[1] = sched.ntp;
-    out3[2] = sched.tm ? sched.tm : lan_default_tm(P.nx, V, sizeof(R) == 8);
+    out3[2] = sched.tm;
     return true;
   }
   void set_schedule(const int32_t* in3) override;

@@ -140,6 +140,7 @@ EnsembleT<R>::EnsembleT(int n, const meu_params* ps, int flags) {
     MEU_CUDA(cudaStreamCreateWithFlags(&b.bst, cudaStreamNonBlocking));
     MEU_CUDA(cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming));
     MEU_CUDA(cudaMalloc(&b.dA, sizeof(LanFusedArgs<R>) * b.idx.size()));
+    b.sched = lan_default(b.N, b.V, sizeof(R) == 8);
   }
   if (persist) {
     // one schedule for every size: the persistent kernel's
@@ -401,10 +402,9 @@ void EnsembleT<R>::schedule(int m, int32_t* out) const {
   if (m < 0 || m >= members) throw CudaError("member index out of range", MEU_ERR_BADARG);
   const auto& b = bk[bucket_of[m]];
   const LanSched& s = b.sched;
-  const int tm = s.tm ? s.tm : lan_default_tm(b.N, b.V, sizeof(R) == 8);
   out[0] = s.pv;
   out[1] = s.ntp;
-  out[2] = tm;
+  out[2] = s.tm;
   out[3] = bucket_of[m];
 }
 

@@ -89,7 +89,7 @@ struct LanFusedArgs {
 // Schedule of the fused kernels: radix plan variant (fz::rplan), threads of the
 // plane kernels, column tile width (complex columns per column-kernel block).
 struct LanSched {
-  int pv = 0, ntp = 512, tm = 0;  // tm = 0: lan_default_tm
+  int pv = 0, ntp = 512, tm = 0;  // of a handle: lan_default
 };
 // Column tile of a handle that sets none.  The column kernels are bound by latency, so more and
 // smaller blocks win until a tile's runs in global memory (tm complex) get short.  Measured on the
@@ -103,6 +103,21 @@ struct LanSched {
 inline int lan_default_tm(int N, int V, bool f64) {
   if (f64) return (N <= 48 && V >= 3) || (N <= 32 && V >= 2) ? 4 : 8;
   return V == 1 ? 16 : 8;
+}
+// Schedule of a handle that sets none.  The radix plan and the plane threads, us per step:
+//  128^3, two or more variants: plan 2 (16 8, one stage less than 8 4 4) against plan 0, with the
+//   column tiles above: FP32 120.0 / 125.6, 169.7 / 175.6, 213.6 / 220.7 for two, three and four
+//   variants, FP64 211.6 / 216.9, 299 / 320, 411 / 439.  One variant (94.4 / 94.0) and the
+//   shorter grids (0 to 30% slower) keep plan 0;
+//  96^3 FP32, one variant: 256 plane threads 60.3, 512 75.1: the 96 planes of a pass leave SMs
+//   idle either way, and the smaller blocks shorten what each waits for at its barriers.  Other
+//   grids gain at most 3% from 256 or lose up to 40%.
+inline LanSched lan_default(int N, int V, bool f64) {
+  LanSched s;
+  s.tm = lan_default_tm(N, V, f64);
+  if (N == 128 && V >= 2) s.pv = 2;
+  if (!f64 && N == 96 && V == 1) s.ntp = 256;
+  return s;
 }
 
 enum LanQ : int {

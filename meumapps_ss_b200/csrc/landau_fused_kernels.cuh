@@ -1372,7 +1372,7 @@ template <typename R, int N, int TM> constexpr bool tm_ok() { return (N * (N / 2
 // s names no instantiated variant.
 template <typename R, int N, int V, typename Fn>
 bool with_sched_v(const LanSched& s, Fn&& f) {
-  const int tm = s.tm ? s.tm : lan_default_tm(N, V, sizeof(R) == 8);
+  const int tm = s.tm;
   auto pick_tm = [&](auto pv_c, auto ntp_c) -> bool {
     constexpr int PV = decltype(pv_c)::value, NTP = decltype(ntp_c)::value;
     if (tm == tm_wide<R>()) {

@@ -111,3 +111,56 @@ def test_kks_fp32_one_variant_against_fp64():
     bound = 64 * 2.0 ** -24
     assert np.linalg.norm(c32 - c64) <= bound * np.linalg.norm(c64)
     assert np.linalg.norm(f32 - f64) <= bound * np.linalg.norm(f64)
+
+
+def _landau_128(nvar, precision, kappa=1.0, n=128):
+    eig = [[0.01] * 3] if nvar == 1 else CF.tetragonal_variants(0.02, -0.005, nvar)
+    p = CF.landau_params(n, nvar, eig, dt=0.005, cross_w=0.5 if nvar > 1 else 0.0, precision=precision,
+                         kappa_c=kappa, kappa_eta=kappa)
+    return (p,) + _fields(p, 31)
+
+
+@pytest.mark.parametrize("nvar,precision", [(2, P.PREC_F64), (3, P.PREC_F32), (4, P.PREC_F64)])
+def test_default_plan_of_128_equals_plan_0(nvar, precision):
+    # two plans of the same transforms: fields, loss and gradients differ by rounding alone, a few
+    # units of a step's sums per step (64 units in the norms; the gradients' sums cancel, times 100).
+    # Both schedules run the adjoint, each on its own order of the spectra.
+    from meumapps_ss_b200.sim import Simulation
+    p, c, e = _landau_128(nvar, precision)
+    unit = 2.0 ** -24 if precision == P.PREC_F32 else 2.0 ** -53
+    out = []
+    for sched in (None, (0, 512, 16 if precision == P.PREC_F32 else 8)):
+        with Simulation(p) as g:
+            if sched:
+                g.set_schedule(*sched)
+            assert g.schedule[0] == (0 if sched else 2)
+            g.set_fields(c, e)
+            J, gr, ge = g.adjoint(3, 2, 0.9 * c, 0.5 * e)
+        with Simulation(p) as g:
+            if sched:
+                g.set_schedule(*sched)
+            g.set_fields(c, e)
+            g.run(3)
+            out.append((g.get_fields()[:2], J, gr, ge))
+    (fa, Ja, ga, gea), (fb, Jb, gb, geb) = out
+    for a, b in zip(fa, fb):
+        assert np.linalg.norm(a - b) <= 64 * unit * np.linalg.norm(b)
+    assert abs(Ja - Jb) <= 64 * unit * abs(Jb)
+    assert np.linalg.norm(gea - geb) <= 64 * unit * np.linalg.norm(geb)
+    for k in gb:
+        assert abs(ga[k] - gb[k]) <= 6400 * unit * abs(gb[k]), k
+
+
+def test_default_plane_threads_of_96_change_nothing():
+    from meumapps_ss_b200.sim import Simulation
+    p, c, e = _landau_128(1, P.PREC_F32, n=96)
+    out = []
+    for sched in (None, (0, 512, 16)):
+        with Simulation(p) as g:
+            if sched:
+                g.set_schedule(*sched)
+            assert g.schedule == (0, 512 if sched else 256, 16)
+            g.set_fields(c, e)
+            J, gr, ge = g.adjoint(3, 2, 0.9 * c, 0.5 * e)
+            out.append((J, gr, ge))
+    assert np.array_equal(out[0][2], out[1][2]) and out[0][0] == out[1][0] and out[0][1] == out[1][1]
