@@ -184,7 +184,8 @@ int meu_destroy(meu_handle* h);
  * complex columns per column-kernel block.  Handles on the generic path (KKS,
  * heterogeneous or non-cubic Landau) report (radix plan of their power-of-two
  * transforms, 0, column-tile factor 1 or 2); MEU_FLAG_AUTOTUNE picks both by
- * timing at meu_create. */
+ * timing at meu_create; their default (0, 0, 1) lets a rule choose the plan and
+ * tile of each y and z pass. */
 int meu_schedule(meu_handle* h, int32_t* out3);
 /* Choose the schedule (same three values) of a fused Landau handle before its
  * first meu_set_fields; MEU_ERR_UNSUPPORTED if the grid and precision have no
@@ -200,7 +201,7 @@ int meu_set_schedule(meu_handle* h, const int32_t* in3);
  *   loss = 1/(2 Nx Ny Nz) sum_x [ (eta_T - eta*)^2 + (c_T - c*)^2 ]
  * with its derivatives computed by the hand-written adjoint of the step
  * (checkpoints of the state every checkpoint_every steps, recomputation of
- * each segment in the reverse sweep):
+ * each segment but the last in the reverse sweep):
  *   dparams[0] = dJ/dbeta   (grad_coeff of eta scaled by beta, at beta = 1)
  *   dparams[1] = dJ/dkappa_c
  *   dparams[2] = dJ/db_mob  (L)
@@ -209,8 +210,8 @@ int meu_set_schedule(meu_handle* h, const int32_t* in3);
  *   dphi0      = dJ/deta_0 (layout as phi; may be NULL)
  * cons_target and phi_target hold c* and eta* (layouts as meu_set_fields).
  * With several order parameters the loss sums (eta_v - eta_v*)^2 over them.
- * Fused Landau handles with 1 to 4 order parameters on the default schedule only
- * (MEU_ERR_UNSUPPORTED otherwise).  The reference has no adjoint. */
+ * Fused Landau handles with 1 to 4 order parameters, on the default schedule or on
+ * (0, 512, 16 FP32 / 8 FP64) only (MEU_ERR_UNSUPPORTED otherwise).  The reference has no adjoint. */
 int meu_adjoint(meu_handle* h, int32_t nsteps, int32_t checkpoint_every, const double* cons_target,
                 const double* phi_target, double* loss, double* dparams, double* dphi0);
 

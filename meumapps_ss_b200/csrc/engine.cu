@@ -444,7 +444,7 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
   MEU_CUDA(cudaMemset(el_ticket, 0, sizeof(unsigned)));
   MEU_CUDA(cudaHostAlloc((void**)&h_ctl, sizeof(ElCtl), cudaHostAllocDefault));
   dK = dalloc<DevConst>(1);
-  MEU_CUDA(cudaHostAlloc((void**)&h_results, sizeof(double) * (Q_TOTAL + PIN_ROWS * Q_STEP_COUNT), cudaHostAllocDefault));
+  MEU_CUDA(cudaHostAlloc((void**)&h_hist, sizeof(double) * PIN_ROWS * Q_STEP_COUNT, cudaHostAllocDefault));
   MEU_CUDA(cudaHostAlloc((void**)&h_err, sizeof(int), cudaHostAllocDefault));
   int ops[Q_TOTAL];
   for (int q = 0; q < Q_TOTAL; ++q) ops[q] = 0;
@@ -719,7 +719,7 @@ Engine<R>::~Engine() {
   drop_graphs();
   prof.reset();
   for (void* q : allocs) cudaFree(q);
-  if (h_results) cudaFreeHost(h_results);
+  if (h_hist) cudaFreeHost(h_hist);
   if (h_err) cudaFreeHost(h_err);
   if (h_ctl) cudaFreeHost(h_ctl);
   for (int b = 0; b < 2; ++b) {
@@ -1470,7 +1470,7 @@ void Engine<R>::flush_hist(meu_diag* diag) {
     MEU_CUDA(cudaMemcpyAsync(h.data(), hist, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
     MEU_CUDA(cudaStreamSynchronize(st));
   }
-  const double* rows = hist_pinned ? h_results + Q_TOTAL : h.data();
+  const double* rows = hist_pinned ? h_hist : h.data();
   hist_pinned = false;
   const double sn3 = (double)n3;
   const bool lan = P.model == MEU_MODEL_LANDAU;
@@ -1516,7 +1516,7 @@ void Engine<R>::queue_flush(cudaStream_t s) {
   MEU_CUDA(cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   hist_pinned = hist_n > 0 && hist_n <= PIN_ROWS;
   if (hist_pinned)
-    MEU_CUDA(cudaMemcpyAsync(h_results + Q_TOTAL, hist, sizeof(double) * (size_t)hist_n * Q_STEP_COUNT,
+    MEU_CUDA(cudaMemcpyAsync(h_hist, hist, sizeof(double) * (size_t)hist_n * Q_STEP_COUNT,
                              cudaMemcpyDeviceToHost, s));
 }
 template <typename R>

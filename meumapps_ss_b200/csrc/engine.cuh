@@ -317,7 +317,7 @@ class Engine : public EngineBase {
     *fc = nullptr, *el_en = nullptr, *strain = nullptr, *xs = nullptr;
   C *sp = nullptr, *uk = nullptr;
   int NS = 0, NWR = 0;
-  double *partials = nullptr, *results = nullptr, *h_results = nullptr;
+  double *partials = nullptr, *results = nullptr, *h_hist = nullptr;
   int* d_ops = nullptr;
   int* d_err = nullptr;
   int* h_err = nullptr;
@@ -465,7 +465,7 @@ class Engine : public EngineBase {
   void flush_hist(meu_diag* diag);
   static constexpr int HIST_MAX = 4096;
   double* hist = nullptr;  // per-step reductions [HIST_MAX][Q_STEP_COUNT]
-  // rows that fit the pinned copy behind h_results (a longer call copies its own)
+  // rows that fit the pinned copy h_hist (a longer call copies its own)
   static constexpr int PIN_ROWS = 128;
   bool hist_pinned = false;  // the pinned copy holds rows 0 .. hist_n - 1
   double* cmean_acc = nullptr;

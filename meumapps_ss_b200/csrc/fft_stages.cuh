@@ -1,6 +1,6 @@
 // fft_stages.cuh -- compile-time radix stages with caller-supplied element access,
 // shared by the generic transforms (fft.cu) and the fused elastic row kernel
-// (el_rows.cu).
+// (el_rows.cuh).
 #pragma once
 #include "fft.cuh"
 #include "fused.cuh"
