@@ -52,6 +52,33 @@ struct CudaError : std::runtime_error {
 
 #define MEU_CHECK_LAUNCH() MEU_CUDA(cudaGetLastError())
 
+// Chained launches of the generic step (programmatic dependent launch): the grid's blocks may be
+// placed while the last blocks of the kernel before it run, and stand at dep_enter, the kernel's
+// first statement, until that kernel has completed and its writes are visible.  The release comes
+// after the wait, so when a chained kernel is placed, everything before its predecessor is
+// complete.  Such kernels read what another kernel writes through pointers without __restrict__:
+// a read-only load must not move above the wait.
+#ifdef __CUDACC__
+__device__ __forceinline__ void dep_enter() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+template <typename... P, typename... Args>
+void launch_dep(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  MEU_CUDA(cudaLaunchKernelEx(&cfg, k, P(args)...));
+}
+#endif
+
 inline unsigned grid_for(int64_t n, int block, int64_t cap = 148 * 16) {
   int64_t g = (n + block - 1) / block;
   if (g > cap) g = cap;

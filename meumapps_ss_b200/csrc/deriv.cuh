@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(NT) k_axis_c(const __grid_constant__ AxisArgs<
   extern __shared__ __align__(16) unsigned char smraw[];
   C* buf = (C*)smraw;  // element e of column l at e * TM + l
   C* lb = buf + L * TM;
+  dep_enter();
   const int tiles = (inner + TM - 1) / TM, o = blockIdx.x / tiles, c0 = (blockIdx.x - o * tiles) * TM;
   const int nc = min(TM, inner - c0), v = blockIdx.y;
   const int64_t at = o * ostride + c0;  // in pairs
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(NT) k_axis_x(const __grid_constant__ AxisArgs<
   extern __shared__ __align__(16) unsigned char smraw[];
   C* buf = (C*)smraw;
   C* lb = buf + N * ES;
+  dep_enter();
   const int v = blockIdx.y;
   const int64_t row0 = (int64_t)blockIdx.x * (2 * NL);
   const int nr = (int)min((int64_t)(2 * NL), nrows - row0);
@@ -266,6 +268,7 @@ __global__ void __launch_bounds__(ZNT) k_z_div(const __grid_constant__ ZDivArgs<
   using TL = fz::StageOf<L, NS - 1, ZPV>;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* buf = (C*)smraw;
+  dep_enter();
   const int64_t inner = A.inner;
   const int c0 = blockIdx.x * TM, nc = min(TM, A.inner - c0), v = blockIdx.y;
   C* sp = A.sp + v * A.stride + c0;
@@ -334,7 +337,7 @@ void launch_c(const AxisArgs<R>& A, int nf, int outer, int inner, int64_t ostrid
   const size_t sm = sizeof(C) * (size_t)L * TM * (A.lap ? 2 : 1);
   auto fn = A.lap ? k_axis_c<R, L, true> : k_axis_c<R, L, false>;
   if ((int)sm > smem_optin((const void*)fn)) throw CudaError("derivative tile exceeds shared memory", MEU_ERR_UNSUPPORTED);
-  fn<<<dim3((unsigned)(outer * ((inner + TM - 1) / TM)), nf), NT, sm, st>>>(A, inner, ostride, (const C*)tw);
+  launch_dep(fn, dim3((unsigned)(outer * ((inner + TM - 1) / TM)), nf), NT, sm, st, A, inner, ostride, (const C*)tw);
 }
 template <typename R, int N>
 void launch_x(const AxisArgs<R>& A, int nf, int64_t nrows, const void* tw, cudaStream_t st) {
@@ -343,7 +346,7 @@ void launch_x(const AxisArgs<R>& A, int nf, int64_t nrows, const void* tw, cudaS
   const size_t sm = sizeof(C) * (size_t)N * (NL | 1) * (A.lap ? 2 : 1);
   auto fn = A.lap ? k_axis_x<R, N, true> : k_axis_x<R, N, false>;
   if ((int)sm > smem_optin((const void*)fn)) throw CudaError("derivative rows exceed shared memory", MEU_ERR_UNSUPPORTED);
-  fn<<<dim3((unsigned)((nrows + 2 * NL - 1) / (2 * NL)), nf), NT, sm, st>>>(A, nrows, (const C*)tw);
+  launch_dep(fn, dim3((unsigned)((nrows + 2 * NL - 1) / (2 * NL)), nf), NT, sm, st, A, nrows, (const C*)tw);
 }
 template <typename R, int L>
 void launch_z(const ZDivArgs<R>& A, int nf, const void* tw, cudaStream_t st) {
@@ -352,7 +355,7 @@ void launch_z(const ZDivArgs<R>& A, int nf, const void* tw, cudaStream_t st) {
   const size_t sm = sizeof(C) * (size_t)L * TM;
   auto fn = A.state ? k_z_div<R, L, true> : k_z_div<R, L, false>;
   if ((int)sm > smem_optin((const void*)fn)) throw CudaError("z tile exceeds shared memory", MEU_ERR_UNSUPPORTED);
-  fn<<<dim3((unsigned)((A.inner + TM - 1) / TM), nf), ZNT, sm, st>>>(A, (const C*)tw);
+  launch_dep(fn, dim3((unsigned)((A.inner + TM - 1) / TM), nf), ZNT, sm, st, A, (const C*)tw);
 }
 
 }  // namespace dv

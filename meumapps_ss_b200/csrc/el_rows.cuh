@@ -258,8 +258,8 @@ __device__ __forceinline__ void polarise(const ElxGen& E, W cfac, R (*g)[2], con
 // inverse transform).
 template <typename R, int N, typename W, typename COEF>
 __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<COEF>()>::BLOCKS))
-    k_el_rows(cplx<R>* __restrict__ sp, int64_t nk, const R* __restrict__ pphi, int64_t n3, int64_t nrows,
-              const cplx<R>* __restrict__ tw, const __grid_constant__ COEF E, const double* __restrict__ cfac_p, int* err) {
+    k_el_rows(cplx<R>* sp, int64_t nk, const R* pphi, int64_t n3, int64_t nrows,
+              const cplx<R>* __restrict__ tw, const __grid_constant__ COEF E, const double* cfac_p, int* err) {
   using C = cplx<R>;
   using G = Geo<R, N, is_gen<COEF>()>;
   constexpr int NR = G::NR, NS = fz::rplan(N, PV).ns, NXH = N / 2 + 1, NT = G::NT;
@@ -270,6 +270,7 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
   R* pbuf = (R*)(smraw + (G::line_bytes + 15) / 16 * 16);
   const int64_t row0 = (int64_t)blockIdx.x * NR;
   const int nr = (int)min((int64_t)NR, nrows - row0);
+  dep_enter();
   prefetch<R, N, G>(pbuf, pphi, E.nvar, n3, row0, nr);
   fz::cp_async_commit();
   const W cfac = cfac_p ? (W)*cfac_p : (W)1;
@@ -518,8 +519,8 @@ void launch_rows(const ElRowsArgs<R>& a, const COEF& E) {
   const size_t sm = (G::line_bytes + 15) / 16 * 16 + sizeof(R) * (size_t)E.nvar * G::NR * G::PS;
   auto fn = k_el_rows<R, N, W, COEF>;
   if ((int)sm > smem_optin((const void*)fn)) throw CudaError("fused elastic rows exceed shared memory", MEU_ERR_UNSUPPORTED);
-  fn<<<(unsigned)((a.nrows + G::NR - 1) / G::NR), G::NT, sm, a.st>>>(a.sp, a.nk, a.pphi, a.n3, a.nrows, (const cplx<R>*)a.tw,
-                                                                 E, a.cfac, a.err);
+  launch_dep(fn, dim3((unsigned)((a.nrows + G::NR - 1) / G::NR)), G::NT, sm, a.st, a.sp, a.nk, a.pphi, a.n3, a.nrows,
+             (const cplx<R>*)a.tw, E, a.cfac, a.err);
 }
 template <typename R, int N, typename COEF>
 void launch_ener(const ElRowsArgs<R>& a, const COEF& E, const R* phi, const DevConst* K, R* el_en, R* elg,

@@ -127,8 +127,8 @@ __device__ __forceinline__ void stages6(C* buf, const C* tw) {
 
 template <typename R, int L>
 __global__ void __launch_bounds__((threads<R, L>()), (min_blocks<R, L>()))
-    k_el_z(cplx<R>* __restrict__ sp, cplx<R>* __restrict__ uk, int64_t nk, const cplx<R>* __restrict__ tw,
-           const __grid_constant__ ElzCoef E, double* __restrict__ part) {
+    k_el_z(cplx<R>* sp, cplx<R>* uk, int64_t nk, const cplx<R>* __restrict__ tw,
+           const __grid_constant__ ElzCoef E, double* part) {
   using C = cplx<R>;
   constexpr int TM = cols<R, L>(), NT = threads<R, L>(), NS = fz::rplan(L, PV).ns;
   using A = Tile<C, TM>;
@@ -155,6 +155,7 @@ __global__ void __launch_bounds__((threads<R, L>()), (min_blocks<R, L>()))
   }
   const int64_t inner = E.inner;
   C* src = sp + c0;
+  dep_enter();
   stage6<C, L, 0, TM, NT, true, true, false>(tw, buf, src, inner, nk, nc);
   __syncthreads();
   stages6<C, L, TM, NT, true, 1, NS>(buf, tw);
@@ -265,8 +266,7 @@ void launch(cplx<R>* sp, cplx<R>* uk, int64_t nk, const void* tw, const ElzCoef&
   constexpr size_t sm = smem_bytes<R, L>();
   const int blocks = (E.inner + cols<R, L>() - 1) / cols<R, L>();
   if ((int)sm > smem_optin((const void*)k_el_z<R, L>)) throw CudaError("elastic z tile exceeds shared memory", MEU_ERR_UNSUPPORTED);
-  k_el_z<R, L><<<blocks, threads<R, L>(), sm, st>>>(sp, uk, nk, (const cplx<R>*)tw, E, part);
-
+  launch_dep(k_el_z<R, L>, dim3(blocks), threads<R, L>(), sm, st, sp, uk, nk, (const cplx<R>*)tw, E, part);
 }
 
 }  // namespace elz

@@ -132,8 +132,9 @@ __device__ void el_control(const ElCtlArgs& A, const double* sums) {
 }
 // the six convergence sums from k_el_z's block partials, in a fixed order (block q sums q);
 // the last block to finish runs the control
-__global__ void __launch_bounds__(1024) k_el_zsum(const double* __restrict__ part, int nblk, double* out, unsigned* ticket,
+__global__ void __launch_bounds__(1024) k_el_zsum(const double* part, int nblk, double* out, unsigned* ticket,
                                                   const __grid_constant__ ElCtlArgs A) {
+  dep_enter();
   const double* p = part + (int64_t)blockIdx.x * nblk;
   double acc = 0;
   for (int i = threadIdx.x; i < nblk; i += blockDim.x) acc += p[i];
@@ -1033,7 +1034,7 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
           if (!elz_q_checked && i == 0) KLAUNCH("el_qcheck", 0.0, k_el_qcheck<<<gridk(), 256, 0, st>>>(dK, d_err));
           KLAUNCH("el_z", 18.0 * nk * sizeof(C), el_z_launch<R>(*fft, S6.p[0], uk, elz, elz_part, st));
           KLAUNCH("finalize", 48.0 * elz_blocks,
-                  k_el_zsum<<<6, 1024, 0, st>>>(elz_part, elz_blocks, results + Q_ERR0, el_ticket, ca));
+                  launch_dep(k_el_zsum, dim3(6), 1024, 0, st, elz_part, elz_blocks, results + Q_ERR0, el_ticket, ca));
         } else {
           fft->pass_z<R>(S6, 6, true, st);
           KLAUNCH("el_k", 18.0 * nk * sizeof(C), k_el_k<R><<<g_el_k, RED_THREADS, 0, st>>>(dK, S6, uk, partials, d_err));

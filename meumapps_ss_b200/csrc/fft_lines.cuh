@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(256) k_cols_s(PtrList<cplx<R>> in, PtrList<cpl
   static_assert(NS >= 2, "first and last stage must differ");
   extern __shared__ __align__(16) unsigned char smraw[];
   C* buf = (C*)smraw;
+  dep_enter();
   const int tiles = (inner + TM - 1) / TM;
   const int o = blockIdx.x / tiles, t = blockIdx.x - o * tiles;
   const int c0 = t * TM, nc = min(TM, inner - c0);
@@ -198,7 +199,7 @@ bool cols_launch(int nf, int outer, int inner, int64_t ostride, const PtrList<cp
   const size_t sm = (size_t)LL * TM * sizeof(C);
   set_smem<R>((const void*)k_cols_s<R, FWD, LL, TM, PV>, sm);
   const dim3 g((unsigned)(outer * ((inner + TM - 1) / TM)), nf);
-  k_cols_s<R, FWD, LL, TM, PV><<<g, 256, sm, st>>>(in, out, inner, ostride, (const C*)tw, scale);
+  launch_dep(k_cols_s<R, FWD, LL, TM, PV>, g, 256, sm, st, in, out, inner, ostride, (const C*)tw, scale);
   return true;
 }
 // lengths with factors 3 (radix plan 3); false when L has no such kernel
