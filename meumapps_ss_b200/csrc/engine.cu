@@ -29,7 +29,8 @@ static bool ortho6(const double* c) {
 }
 
 // Fixed-order finalisation: block q reduces partials[q*PSTRIDE .. + nb[q]) with ops[q].
-__global__ void k_finalize(const double* __restrict__ partials, NbList nb, const int* __restrict__ ops, double* out) {
+__global__ void k_finalize(const double* partials, NbList nb, const int* __restrict__ ops, double* out) {
+  dep_enter();
   const int q = blockIdx.x, op = ops[q];
   double acc = op == 0 ? 0.0 : op == 1 ? -1.0e308 : 1.0e308;
   for (int i = threadIdx.x; i < nb.nb[q]; i += blockDim.x) {
@@ -749,7 +750,7 @@ void Engine<R>::finalize(int q0, int nq, double* out, const int* nbs) {
   NbList nb;
   for (int q = 0; q < nq; ++q) nb.nb[q] = nbs ? nbs[q] : (q0 + q == Q_ELEN && el_fused_rows) ? PSTRIDE : RED_BLOCKS;
   KLAUNCH("finalize", 8.0 * nq * RED_BLOCKS,
-          k_finalize<<<nq, 256, 0, st>>>(partials + (int64_t)q0 * PSTRIDE, nb, d_ops + q0, out ? out : results + q0));
+          launch_dep(k_finalize, dim3(nq), 256, 0, st, partials + (int64_t)q0 * PSTRIDE, nb, d_ops + q0, out ? out : results + q0));
 }
 
 // ---- host-side AoS conversion in chunks through the staging buffer
@@ -1451,7 +1452,7 @@ void Engine<R>::landau_step(meu_diag* d) {
 template <typename R>
 void Engine<R>::end_step(meu_diag* d, int clip) {
   KLAUNCH("stats", (double)(E + V * (clip ? 2 : 1)) * n3 * sizeof(R),
-          k_stats<R><<<RED_BLOCKS, RED_THREADS, 0, st>>>(dK, c, phi, clip, partials));
+          launch_dep(k_stats<R>, dim3(RED_BLOCKS), RED_THREADS, 0, st, dK, c, phi, clip, partials));
   // this step's reductions go straight into the device history, read once per meu_run
   finalize(0, Q_STEP_COUNT, hist + (int64_t)hist_n * Q_STEP_COUNT);
   hist_step[hist_n] = step;

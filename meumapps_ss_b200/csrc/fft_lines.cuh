@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(256) k_rows_r2c_s(PtrList<const R> in, PtrList
   static_assert(NS >= 2, "first and last stage must differ");
   extern __shared__ __align__(16) unsigned char smraw[];
   C* buf = (C*)smraw;
+  dep_enter();
   const int64_t row0 = (int64_t)blockIdx.x * NR;
   const int nr = (int)min((int64_t)NR, nrows - row0);
   const C* src = (const C*)(in.p[blockIdx.y] + row0 * (2 * L));
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(256) k_rows_c2r_s(PtrList<const cplx<R>> in, P
   static_assert(NS >= 2, "first and last stage must differ");
   extern __shared__ __align__(16) unsigned char smraw[];
   C* buf = (C*)smraw;
+  dep_enter();
   const int64_t row0 = (int64_t)blockIdx.x * NR;
   const int nr = (int)min((int64_t)NR, nrows - row0);
   const C* src = in.p[blockIdx.y] + row0 * NXH;
@@ -183,12 +185,12 @@ bool rows_launch(bool fwd, int nf, int64_t nrows, const void* in, const void* ou
   const dim3 g((unsigned)((nrows + NR - 1) / NR), nf);
   if (fwd) {
     set_smem<R>((const void*)k_rows_r2c_s<R, LL, PV>, sm);
-    k_rows_r2c_s<R, LL, PV><<<g, 256, sm, st>>>(*(const PtrList<const R>*)in, *(const PtrList<C>*)out, nrows,
-                                                 (const C*)tw, (const C*)post);
+    launch_dep(k_rows_r2c_s<R, LL, PV>, g, 256, sm, st, *(const PtrList<const R>*)in, *(const PtrList<C>*)out, nrows,
+               (const C*)tw, (const C*)post);
   } else {
     set_smem<R>((const void*)k_rows_c2r_s<R, LL, PV>, sm);
-    k_rows_c2r_s<R, LL, PV><<<g, 256, sm, st>>>(*(const PtrList<const C>*)in, *(const PtrList<R>*)out, nrows,
-                                                 (const C*)tw, (const C*)post);
+    launch_dep(k_rows_c2r_s<R, LL, PV>, g, 256, sm, st, *(const PtrList<const C>*)in, *(const PtrList<R>*)out, nrows,
+               (const C*)tw, (const C*)post);
   }
   return true;
 }

@@ -970,6 +970,7 @@ __global__ void __launch_bounds__(256) k_lan_b(const DevConst* __restrict__ Kp, 
 template <typename R>
 __global__ void __launch_bounds__(RED_THREADS) k_stats(const DevConst* __restrict__ Kp, const R* __restrict__ c,
                                                        R* __restrict__ phi, int clip, double* partials) {
+  dep_enter();  // every field read below is guarded by the loop's bound
   const DevConst& K = *Kp;
   const int64_t n3 = K.n3;
   const int V = K.p.nvar, E = K.p.numel;
