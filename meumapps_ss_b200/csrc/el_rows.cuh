@@ -16,6 +16,8 @@
 // and nothing is permuted; the last inverse stage, the polarisation and the first forward stage
 // run on one butterfly's registers of all six components.
 #pragma once
+#include <type_traits>
+
 #include "engine.cuh"
 #include "fft_stages.cuh"
 #include "step_kernels.cuh"
@@ -535,9 +537,37 @@ void launch_ener(const ElRowsArgs<R>& a, const COEF& E, const R* phi, const DevC
                                          out, eta2, partials, a.err);
 }
 
-}  // namespace elr
+// lengths of the two units of a precision (el_rows_*_a.cu: up to 128, el_rows_*_b.cu: longer)
+template <int... N>
+struct Lengths {};
+using LenA = Lengths<16, 24, 32, 36, 48, 54, 64, 72, 96, 108, 128>;
+using LenB = Lengths<144, 162, 192, 216, 256, 288, 324, 384, 432, 512, 1024>;
+// fn(N as an integral constant) for N = nx; false when the unit has no kernels of that length
+template <int... N, typename FN>
+bool with_length(Lengths<N...>, int nx, FN&& fn) {
+  return ((nx == N && (fn(std::integral_constant<int, N>{}), true)) || ...);
+}
+template <typename R, typename LEN>
+bool rows_unit(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, bool fp64) {
+  return with_length(LEN{}, a.nx, [&](auto n) {
+    constexpr int N = decltype(n)::value;
+    if (!c.prop) return launch_rows<R, N, double, ElxGen>(a, *c.gen);
+    if constexpr (sizeof(R) == 4) {
+      if (fp64) return launch_rows<R, N, double, ElxProp>(a, *c.p64);
+    }
+    launch_rows<R, N, R, ElxCoef<R>>(a, *c.pr);
+  });
+}
+template <typename R, typename LEN>
+bool ener_unit(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, const R* phi, const DevConst* K, R* el_en, R* elg,
+               const EnerOut<R>& out, int eta2, double* partials) {
+  return with_length(LEN{}, a.nx, [&](auto n) {
+    constexpr int N = decltype(n)::value;
+    if (c.prop) launch_ener<R, N, ElenProp>(a, *c.en, phi, K, el_en, elg, out, eta2, partials);
+    else launch_ener<R, N, ElxGen>(a, *c.gen, phi, K, el_en, elg, out, eta2, partials);
+  });
+}
 
-#define MEU_ROWS_A(X) X(16) X(24) X(32) X(36) X(48) X(54) X(64) X(72) X(96) X(108) X(128)
-#define MEU_ROWS_B(X) X(144) X(162) X(192) X(216) X(256) X(288) X(324) X(384) X(432) X(512) X(1024)
+}  // namespace elr
 
 }  // namespace meu
