@@ -149,15 +149,16 @@ __device__ __forceinline__ void prefetch(R* dst, const R* __restrict__ src, int 
     }
 }
 
-// fn(v) for every variant, unrolled (coefficients at fixed parameter addresses) up to four
-template <typename FN>
+// fn(v) for every variant, unrolled (coefficients at fixed parameter addresses) up to four; UN at a
+// time beyond (4 where the order parameters come from global memory: their loads overlap)
+template <int UN, typename FN>
 __device__ __forceinline__ void each_variant(int V, FN&& fn) {
   if (V <= 4) {
 #pragma unroll
     for (int v = 0; v < 4; ++v)
       if (v < V) fn(v);
   } else {
-#pragma unroll 1
+#pragma unroll UN
     for (int v = 0; v < V; ++v) fn(v);
   }
 }
@@ -189,10 +190,10 @@ __device__ __forceinline__ double gen_mix(const ElxGen& E, const R* pp, int64_t 
 // polarisation of two voxels (h = 0, 1) from their engineering strains g[m][h], in place,
 // proportional moduli (C(x) = C_1 / s(x); k_el_x_prop's formula) in the precision W.  Order
 // parameter v of voxel h at pp[v * vs + h * hs].
-template <typename W, typename R>
-__device__ __forceinline__ void polarise(const ElxCoef<W>& E, W cfac, R (*g)[2], const R* pp, int vs, int hs, int* err) {
+template <int UN, typename W, typename R, typename S>
+__device__ __forceinline__ void polarise(const ElxCoef<W>& E, W cfac, R (*g)[2], const R* pp, S vs, int hs, int* err) {
   W e0[2][6] = {}, psum[2] = {0, 0}, sc[2] = {0, 0};
-  each_variant(E.nvar, [&](int v) {
+  each_variant<UN>(E.nvar, [&](int v) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const W q = (W)pp[v * vs + h * hs];
@@ -226,13 +227,13 @@ __device__ __forceinline__ void polarise(const ElxCoef<W>& E, W cfac, R (*g)[2],
 }
 // the same for general moduli with decoupled normal and shear parts (k_el_x<R, true>): the
 // mixed compliance inverted as a 3x3 block and three shears, FP64
-template <typename W, typename R>
-__device__ __forceinline__ void polarise(const ElxGen& E, W cfac, R (*g)[2], const R* pp, int vs, int hs, int* err) {
+template <int UN, typename W, typename R, typename S>
+__device__ __forceinline__ void polarise(const ElxGen& E, W cfac, R (*g)[2], const R* pp, S vs, int hs, int* err) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     double Cm[36], e0[6] = {0, 0, 0, 0, 0, 0};
     gen_mix(E, pp + h * hs, vs, Cm, true);
-    each_variant(E.nvar, [&](int v) {
+    each_variant<UN>(E.nvar, [&](int v) {
       const double q = (double)pp[v * vs + h * hs];
 #pragma unroll
       for (int m = 0; m < 6; ++m) e0[m] += q * E.ep[v][m];
@@ -256,9 +257,9 @@ __device__ __forceinline__ void polarise(const ElxGen& E, W cfac, R (*g)[2], con
 }
 
 // sp: the six row spectra (contiguous, nk apart), in place; E: ElxCoef<W> or ElxGen.  Dynamic
-// shared memory: the lines, then the block's order parameters (cp.async, in flight during the
-// inverse transform).
-template <typename R, int N, typename W, typename COEF>
+// shared memory: the lines, then with STAGE the block's order parameters (cp.async, in flight during
+// the inverse transform); else they are read from global memory where they are used.
+template <typename R, int N, typename W, typename COEF, bool STAGE>
 __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<COEF>()>::BLOCKS))
     k_el_rows(cplx<R>* sp, int64_t nk, const R* pphi, int64_t n3, int64_t nrows,
               const cplx<R>* __restrict__ tw, const __grid_constant__ COEF E, const double* cfac_p, int* err) {
@@ -273,14 +274,18 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
   const int64_t row0 = (int64_t)blockIdx.x * NR;
   const int nr = (int)min((int64_t)NR, nrows - row0);
   dep_enter();
-  prefetch<R, N, G>(pbuf, pphi, E.nvar, n3, row0, nr);
-  fz::cp_async_commit();
+  if constexpr (STAGE) {
+    prefetch<R, N, G>(pbuf, pphi, E.nvar, n3, row0, nr);
+    fz::cp_async_commit();
+  }
   const W cfac = cfac_p ? (W)*cfac_p : (W)1;
   head<R, N, G>(buf, sp, nk, row0, nr, tw);
   __syncthreads();
   stages<R, N, G, true, 1, NS - 1>(buf, tw);
-  fz::cp_async_wait_all();
-  __syncthreads();
+  if constexpr (STAGE) {
+    fz::cp_async_wait_all();
+    __syncthreads();
+  }
   // last inverse stage, polarisation, first forward stage on the registers of one butterfly
 #pragma unroll 1
   for (int t = threadIdx.x; t < NR / 2 * TL::TASKS; t += G::NT) {
@@ -304,7 +309,9 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
       }
       // a row past nr takes the block's first row (it is not stored)
       const int r0 = 2 * i < nr ? 2 * i : 0, r1 = 2 * i + 1 < nr ? 2 * i + 1 : r0;
-      polarise<W>(E, cfac, g, pbuf + r0 * G::PS + n0 + q * (N / TL::R), NR * G::PS, (r1 - r0) * G::PS, err);
+      const int n = n0 + q * (N / TL::R);
+      if constexpr (STAGE) polarise<STAGE ? 1 : 4, W>(E, cfac, g, pbuf + r0 * G::PS + n, NR * G::PS, (r1 - r0) * G::PS, err);
+      else polarise<STAGE ? 1 : 4, W>(E, cfac, g, pphi + (row0 + r0) * N + n, n3, (r1 - r0) * N, err);
 #pragma unroll
       for (int m = 0; m < 6; ++m) x[m][q] = mk(g[m][0], g[m][1]);
     }
@@ -339,11 +346,11 @@ struct EnerVox {
   double sig[6], mat, psum;
 };
 // proportional moduli (k_elener_prop): sigma = C_1 eps / s
-template <typename R>
+template <int UN, typename R, typename S>
 __device__ __forceinline__ void ener_stress(const ElenProp& E, const DevConst&, const double* gam, const R* pp,
-                                            int vs, EnerVox& o, int* err) {
+                                            S vs, EnerVox& o, int* err) {
   double te[6] = {0, 0, 0, 0, 0, 0}, ps = 0, sc = 0, eps[6], em[6];
-  each_variant(E.nvar, [&](int v) {
+  each_variant<UN>(E.nvar, [&](int v) {
     const double q = (double)pp[v * vs];
     ps += q;
     sc += E.av[v] * q;
@@ -375,11 +382,11 @@ __device__ __forceinline__ bool ener_use(const ElenProp& E, const DevConst&, int
 __device__ __forceinline__ const double* ener_tp(const ElenProp& E, const DevConst&, int v) { return E.tp[v]; }
 
 // general moduli with decoupled normal and shear parts (k_elener<R, true>)
-template <typename R>
+template <int UN, typename R, typename S>
 __device__ __forceinline__ void ener_stress(const ElxGen& E, const DevConst& K, const double* gam, const R* pp,
-                                            int vs, EnerVox& o, int* err) {
+                                            S vs, EnerVox& o, int* err) {
   double te[6] = {0, 0, 0, 0, 0, 0}, Cm[36], eps[6];
-  each_variant(E.nvar, [&](int v) {
+  each_variant<UN>(E.nvar, [&](int v) {
     const double q = (double)pp[v * vs];
 #pragma unroll
     for (int m = 0; m < 6; ++m) te[m] += q * E.ep[v][m];  // engineering shear
@@ -408,10 +415,10 @@ __device__ __forceinline__ const double* ener_tp(const ElxGen&, const DevConst& 
 
 // Row blocks of the final strain: x C2R, then elener with the voxels in row order (the last
 // inverse stage stores every voxel at its own place, after a barrier, so that global memory is
-// read and written in rows; order parameters and P by cp.async during the transform); the
-// driving force as EnerOut says.  Grid-stride over row blocks: at most PSTRIDE
+// read and written in rows; with STAGE order parameters and P by cp.async during the transform);
+// the driving force as EnerOut says.  Grid-stride over row blocks: at most PSTRIDE
 // blocks, each one partial of the energy sum.
-template <typename R, int N, typename COEF>
+template <typename R, int N, typename COEF, bool STAGE>
 __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<COEF>()>::BLOCKS))
     k_el_ener(const cplx<R>* __restrict__ sp, int64_t nk, const R* __restrict__ phi, const R* __restrict__ pphi,
               int64_t n3, int64_t nrows, const cplx<R>* __restrict__ tw, const DevConst* __restrict__ Kp,
@@ -420,6 +427,8 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
   using C = cplx<R>;
   using G = Geo<R, N, is_gen<COEF>()>;
   constexpr int NR = G::NR, NS = fz::rplan(N, PV).ns, NT = G::NT, VS = NR * G::PS;
+  using VT = std::conditional_t<STAGE, int, int64_t>;
+  constexpr int UN = STAGE ? 1 : 4;
   using TL = fz::StageOf<N, NS - 1, PV>;
   constexpr int IT = (G::NL * TL::TASKS + NT - 1) / NT;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -431,9 +440,11 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
 #pragma unroll 1
   for (int64_t row0 = (int64_t)blockIdx.x * NR; row0 < nrows; row0 += (int64_t)gridDim.x * NR) {
     const int nr = (int)min((int64_t)NR, nrows - row0);
-    prefetch<R, N, G>(pb, pphi, E.nvar, n3, row0, nr);
-    prefetch<R, N, G>(fb, phi, E.nvar, n3, row0, nr);
-    fz::cp_async_commit();
+    if constexpr (STAGE) {
+      prefetch<R, N, G>(pb, pphi, E.nvar, n3, row0, nr);
+      prefetch<R, N, G>(fb, phi, E.nvar, n3, row0, nr);
+      fz::cp_async_commit();
+    }
     head<R, N, G>(buf, sp, nk, row0, nr, tw);
     __syncthreads();
     stages<R, N, G, true, 1, NS - 1>(buf, tw);
@@ -459,30 +470,31 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
         }
       }
     }
-    fz::cp_async_wait_all();
+    if constexpr (STAGE) fz::cp_async_wait_all();
     __syncthreads();
 #pragma unroll 1
     for (int i = threadIdx.x; i < nr * N; i += G::NT) {
       const int r = i / N, n = i - r * N;
       const int64_t id = (row0 + r) * N + n;
       const R* e = (const R*)(buf + n * G::ES + r / 2 * 6) + (r & 1);
-      const R *pv = pb + r * G::PS + n, *fv = fb + r * G::PS + n;
+      const R *pv = STAGE ? pb + r * G::PS + n : pphi + id, *fv = STAGE ? fb + r * G::PS + n : phi + id;
+      const VT vs = STAGE ? (VT)VS : (VT)n3;
       double gam[6];
 #pragma unroll
       for (int m = 0; m < 6; ++m) gam[m] = (double)e[2 * m];
       EnerVox o;
-      ener_stress(E, K, gam, pv, VS, o, err);
+      ener_stress<UN>(E, K, gam, pv, vs, o, err);
       double en = (1.0 - o.psum) * o.mat, s2 = 0, cv = 0;
       if (out.mode == 3) {
         cv = K.c_mean[0] + (double)out.c[id];
-        each_variant(E.nvar, [&](int v) { s2 += (double)fv[v * VS] * (double)fv[v * VS]; });
+        each_variant<UN>(E.nvar, [&](int v) { s2 += (double)fv[v * vs] * (double)fv[v * vs]; });
       }
-      each_variant(E.nvar, [&](int v) {
-        const double f = (double)fv[v * VS];
+      each_variant<UN>(E.nvar, [&](int v) {
+        const double f = (double)fv[v * vs];
         double eg = 0;
         if (ener_use(E, K, v)) {
           const double elp = ener_ppt(E, K, v, o);
-          en += elp * (double)pv[v * VS];
+          en += elp * (double)pv[v * vs];
           const double* t = ener_tp(E, K, v);
           const double g = o.sig[0] * t[0] + o.sig[1] * t[1] + o.sig[2] * t[2] +
                            2.0 * (o.sig[3] * t[3] + o.sig[4] * t[4] + o.sig[5] * t[5]);
@@ -515,11 +527,25 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
   block_reduce_store(esum, 0, partials + Q_ELEN * PSTRIDE + blockIdx.x);
 }
 
+// Order parameters come through shared memory while that leaves two blocks per SM and more than half
+// of those that the lines alone would; else straight from global memory, so that any number of
+// variants runs on every length.  Staged / direct, us per launch: k_el_rows KKS 64^3 FP64 3
+// variants 20.9 / 23.5, 12 36.4 / 31.0; 512 x 32 x 32 FP64 10 variants 135 / 82; 256 x 128 x 64 FP32 4
+// variants 57 / 66; 1024 x 32 x 16 FP64 3 variants 82 / 73.  k_el_ener, which stages P and the order
+// parameters: KKS 64^3 FP64 6 variants 46.9 / 36.4, 12 169 / 68; 128^3 FP64 3 167 / 196, 6 271 / 266;
+// 512 x 32 x 32 FP64 2 61 / 76, 10 232 / 196; 128 x 128 x 64 FP32 8 99 / 95, 16 234 / 172.
+template <typename R, bool GEN>
+bool stage_pars(size_t lines, size_t pars) {
+  auto blocks = [](size_t sm) { return std::min(Cfg<R, GEN>::BLOCKS, (int)((228 * 1024) / (sm + 1024))); };
+  return blocks(lines + pars) >= 2 && 2 * blocks(lines + pars) > blocks(lines);
+}
 template <typename R, int N, typename W, typename COEF>
 void launch_rows(const ElRowsArgs<R>& a, const COEF& E) {
   using G = Geo<R, N, is_gen<COEF>()>;
-  const size_t sm = (G::line_bytes + 15) / 16 * 16 + sizeof(R) * (size_t)E.nvar * G::NR * G::PS;
-  auto fn = k_el_rows<R, N, W, COEF>;
+  const size_t lines = (G::line_bytes + 15) / 16 * 16, pars = sizeof(R) * (size_t)E.nvar * G::NR * G::PS;
+  const bool stage = stage_pars<R, is_gen<COEF>()>(lines, pars);
+  const size_t sm = lines + (stage ? pars : 0);
+  auto fn = stage ? k_el_rows<R, N, W, COEF, true> : k_el_rows<R, N, W, COEF, false>;
   if ((int)sm > smem_optin((const void*)fn)) throw CudaError("fused elastic rows exceed shared memory", MEU_ERR_UNSUPPORTED);
   launch_dep(fn, dim3((unsigned)((a.nrows + G::NR - 1) / G::NR)), G::NT, sm, a.st, a.sp, a.nk, a.pphi, a.n3, a.nrows,
              (const cplx<R>*)a.tw, E, a.cfac, a.err);
@@ -528,8 +554,10 @@ template <typename R, int N, typename COEF>
 void launch_ener(const ElRowsArgs<R>& a, const COEF& E, const R* phi, const DevConst* K, R* el_en, R* elg,
                  const EnerOut<R>& out, int eta2, double* partials) {
   using G = Geo<R, N, is_gen<COEF>()>;
-  auto fn = k_el_ener<R, N, COEF>;
-  const size_t sm = (G::line_bytes + 15) / 16 * 16 + sizeof(R) * (size_t)(2 * E.nvar) * G::NR * G::PS;
+  const size_t lines = (G::line_bytes + 15) / 16 * 16, pars = sizeof(R) * (size_t)(2 * E.nvar) * G::NR * G::PS;
+  const bool stage = stage_pars<R, is_gen<COEF>()>(lines, pars);
+  const size_t sm = lines + (stage ? pars : 0);
+  auto fn = stage ? k_el_ener<R, N, COEF, true> : k_el_ener<R, N, COEF, false>;
   if ((int)sm > smem_optin((const void*)fn))
     throw CudaError("elastic energy rows exceed shared memory", MEU_ERR_UNSUPPORTED);
   const unsigned blocks = (unsigned)std::min<int64_t>((a.nrows + G::NR - 1) / G::NR, PSTRIDE);
