@@ -527,23 +527,25 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
   block_reduce_store(esum, 0, partials + Q_ELEN * PSTRIDE + blockIdx.x);
 }
 
-// Order parameters come through shared memory while that leaves two blocks per SM and more than half
-// of those that the lines alone would; else straight from global memory, so that any number of
+// Order parameters come through shared memory while that leaves two blocks per SM, for elener (which
+// stages P and the order parameters, and reads them row by row otherwise) also more than half of
+// the blocks that the lines alone would; else straight from global memory, so that any number of
 // variants runs on every length.  Staged / direct, us per launch: k_el_rows KKS 64^3 FP64 3
-// variants 20.9 / 23.5, 12 36.4 / 31.0; 512 x 32 x 32 FP64 10 variants 135 / 82; 256 x 128 x 64 FP32 4
-// variants 57 / 66; 1024 x 32 x 16 FP64 3 variants 82 / 73.  k_el_ener, which stages P and the order
-// parameters: KKS 64^3 FP64 6 variants 46.9 / 36.4, 12 169 / 68; 128^3 FP64 3 167 / 196, 6 271 / 266;
-// 512 x 32 x 32 FP64 2 61 / 76, 10 232 / 196; 128 x 128 x 64 FP32 8 99 / 95, 16 234 / 172.
+// variants 20.9 / 23.5, 12 36.4 / 31.0; 1024 x 32 x 16 FP32 4 variants 32 / 37, 8 49 / 35, FP64 3 82 / 73;
+// 512 x 32 x 32 FP64 10 variants 135 / 82.  k_el_ener: KKS 64^3 FP64 6 variants 46.9 / 36.4, 12
+// 169 / 68; 128^3 FP64 3 167 / 196, 6 271 / 266; 512 x 32 x 32 FP64 2 61 / 76, 10 232 / 196;
+// 128 x 128 x 64 FP32 8 99 / 95, 16 234 / 172.
 template <typename R, bool GEN>
-bool stage_pars(size_t lines, size_t pars) {
+bool stage_pars(size_t lines, size_t pars, bool ener) {
   auto blocks = [](size_t sm) { return std::min(Cfg<R, GEN>::BLOCKS, (int)((228 * 1024) / (sm + 1024))); };
-  return blocks(lines + pars) >= 2 && 2 * blocks(lines + pars) > blocks(lines);
+  const int b = blocks(lines + pars);
+  return b >= 2 && (!ener || 2 * b > blocks(lines));
 }
 template <typename R, int N, typename W, typename COEF>
 void launch_rows(const ElRowsArgs<R>& a, const COEF& E) {
   using G = Geo<R, N, is_gen<COEF>()>;
   const size_t lines = (G::line_bytes + 15) / 16 * 16, pars = sizeof(R) * (size_t)E.nvar * G::NR * G::PS;
-  const bool stage = stage_pars<R, is_gen<COEF>()>(lines, pars);
+  const bool stage = stage_pars<R, is_gen<COEF>()>(lines, pars, false);
   const size_t sm = lines + (stage ? pars : 0);
   auto fn = stage ? k_el_rows<R, N, W, COEF, true> : k_el_rows<R, N, W, COEF, false>;
   if ((int)sm > smem_optin((const void*)fn)) throw CudaError("fused elastic rows exceed shared memory", MEU_ERR_UNSUPPORTED);
@@ -555,7 +557,7 @@ void launch_ener(const ElRowsArgs<R>& a, const COEF& E, const R* phi, const DevC
                  const EnerOut<R>& out, int eta2, double* partials) {
   using G = Geo<R, N, is_gen<COEF>()>;
   const size_t lines = (G::line_bytes + 15) / 16 * 16, pars = sizeof(R) * (size_t)(2 * E.nvar) * G::NR * G::PS;
-  const bool stage = stage_pars<R, is_gen<COEF>()>(lines, pars);
+  const bool stage = stage_pars<R, is_gen<COEF>()>(lines, pars, true);
   const size_t sm = lines + (stage ? pars : 0);
   auto fn = stage ? k_el_ener<R, N, COEF, true> : k_el_ener<R, N, COEF, false>;
   if ((int)sm > smem_optin((const void*)fn))
