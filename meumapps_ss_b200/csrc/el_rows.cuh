@@ -532,9 +532,9 @@ __global__ void __launch_bounds__((Cfg<R, is_gen<COEF>()>::NT), (Cfg<R, is_gen<C
 // the blocks that the lines alone would; else straight from global memory, so that any number of
 // variants runs on every length.  Staged / direct, us per launch: k_el_rows KKS 64^3 FP64 3
 // variants 20.9 / 23.5, 12 36.4 / 31.0; 1024 x 32 x 16 FP32 4 variants 32 / 37, 8 49 / 35, FP64 3 82 / 73;
-// 512 x 32 x 32 FP64 10 variants 135 / 82.  k_el_ener: KKS 64^3 FP64 6 variants 46.9 / 36.4, 12
-// 169 / 68; 128^3 FP64 3 167 / 196, 6 271 / 266; 512 x 32 x 32 FP64 2 61 / 76, 10 232 / 196;
-// 128 x 128 x 64 FP32 8 99 / 95, 16 234 / 172.
+// 512 x 32 x 32 FP64 10 variants 135 / 82.  k_el_ener: KKS 64^3 FP64 12 169 / 68; 128^3 FP64 3
+// 167 / 196; 512 x 32 x 32 FP64 2 61 / 76, 10 232 / 196; 128 x 128 x 64 FP32 16 234 / 172.  With three
+// blocks left of four either wins (FP64 64^3 6 variants 46.9 / 36.4, 128^3 6 271 / 266).
 template <typename R, bool GEN>
 bool stage_pars(size_t lines, size_t pars, bool ener) {
   auto blocks = [](size_t sm) { return std::min(Cfg<R, GEN>::BLOCKS, (int)((228 * 1024) / (sm + 1024))); };
@@ -577,15 +577,24 @@ template <int... N, typename FN>
 bool with_length(Lengths<N...>, int nx, FN&& fn) {
   return ((nx == N && (fn(std::integral_constant<int, N>{}), true)) || ...);
 }
+// FP32 fields with proportional moduli form the polarisation in FP64, but for rows of 64 to 1024 in
+// powers of two, which take it in the field precision after a step's first iteration.  It is a
+// difference of stresses, so FP32 leaves 2^-24 times the larger ones in it: strains against FP64 at 48 x 12 x 16 4.4 units of 2^-24 from FP64, 5.0 from
+// FP32; under a mean strain of 0.3 53 and 103.  FP64 / FP32, us per launch: 48^3 one variant
+// 15.0 / 14.2, 96^3 two 35.6 / 32.6, 108 x 144 x 96 three 54.4 / 49.2.
+template <typename R, int N>
+constexpr bool field_polarisation() {
+  return sizeof(R) == 8 || (N >= 64 && (N & (N - 1)) == 0);
+}
 template <typename R, typename LEN>
 bool rows_unit(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, bool fp64) {
   return with_length(LEN{}, a.nx, [&](auto n) {
     constexpr int N = decltype(n)::value;
     if (!c.prop) return launch_rows<R, N, double, ElxGen>(a, *c.gen);
-    if constexpr (sizeof(R) == 4) {
-      if (fp64) return launch_rows<R, N, double, ElxProp>(a, *c.p64);
+    if constexpr (field_polarisation<R, N>()) {
+      if (sizeof(R) == 8 || !fp64) return launch_rows<R, N, R, ElxCoef<R>>(a, *c.pr);
     }
-    launch_rows<R, N, R, ElxCoef<R>>(a, *c.pr);
+    if constexpr (sizeof(R) == 4) launch_rows<R, N, double, ElxProp>(a, *c.p64);
   });
 }
 template <typename R, typename LEN>

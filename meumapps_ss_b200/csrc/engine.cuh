@@ -143,7 +143,8 @@ struct ElRowsCoef {
   const ElenProp* en;
   const ElxGen* gen;
 };
-// false: no kernel for nx (a: up to 128, b: longer).  fp64: the polarisation in FP64.
+// false: no kernel for nx (a: up to 128, b: longer).  fp64: the polarisation in FP64 whatever the
+// length (it is for most lengths, see field_polarisation).
 template <typename R>
 bool el_rows_a(const ElRowsArgs<R>& a, const ElRowsCoef<R>& c, bool fp64);
 template <typename R>

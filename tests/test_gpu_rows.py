@@ -76,3 +76,27 @@ def test_long_rows_and_many_variants_match_oracle(oracle, nvar, moduli, box):
 def test_kks_many_variants_match_oracle(oracle, nvar, box):
     p, c, e = _kks(*box, nvar)
     _compare(oracle, p, c, e, 2)
+
+
+@pytest.mark.parametrize("box", [(16, 16, 18), (48, 12, 16), (54, 9, 8), (108, 8, 6), (144, 8, 6), (384, 4, 6)])
+def test_fp32_polarisation_is_formed_in_fp64(box):
+    # General moduli form the polarisation in FP64 from FP32 fields.  The same moduli, proportional but
+    # for 1e-9, must leave the same error against FP64, up to the scatter of a few thousand roundings
+    # (a quarter).  The mean strain makes the polarisation a difference of large stresses: formed
+    # in FP32 its error is 1.5 to 1.9 times as large.  Eight iterations in every run.
+    p, c, e = _hetero(*box, 2, "proportional")
+    p.el_min_iter = p.el_max_iter = 8
+    for m in range(3):
+        p.e_mean[m] = 0.3
+    _, (_, _, n64, u64) = _run(p, c, e, 1)
+    err = []
+    for scale in (1.0, 1.0 + 1e-9):
+        q = p.copy()
+        q.precision = P.PREC_F32
+        m = CF.cubic(375.0 * scale, 225.0, 150.0)
+        q.set_matrix("cela", 1, m)
+        q.set_matrix("sela", 1, np.linalg.inv(m))
+        d, (_, _, n32, u32) = _run(q, c, e, 1)
+        assert list(d["el_iters"]) == [8]
+        err.append((np.linalg.norm(u32[3:] - u64[3:]), np.linalg.norm(n32 - n64)))
+    assert err[0][0] <= 1.25 * err[1][0] and err[0][1] <= 1.25 * err[1][1]
