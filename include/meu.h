@@ -184,14 +184,16 @@ int meu_destroy(meu_handle* h);
  * complex columns per column-kernel block.  Handles on the generic path (KKS,
  * heterogeneous or non-cubic Landau) report (radix plan of their power-of-two
  * transforms, 0, column-tile factor 1 or 2); MEU_FLAG_AUTOTUNE picks both by
- * timing at meu_create; their default (0, 0, 1) lets a rule choose the plan and
- * tile of each y and z pass. */
+ * timing at meu_create.  A generic handle that has chosen none, and one for which
+ * the autotuner kept it, takes plan and tile of each y and z pass from a rule on
+ * its length, direction and precision, and reports (0, 0, 1). */
 int meu_schedule(meu_handle* h, int32_t* out3);
 /* Choose the schedule (same three values) of a fused Landau handle before its
  * first meu_set_fields; MEU_ERR_UNSUPPORTED if the grid and precision have no
  * such variant (the variants: radix plan 0, 1 or 2, 512 or 256 plane threads,
  * column tile 16 or 8 in FP32, 8 or 4 in FP64 where the tiles fit).  A generic
- * handle takes (0 or 2, 0, 1 or 2) at any time. */
+ * handle takes (0 or 2, 0, 1 or 2) at any time and then runs that plan and tile in
+ * every pass. */
 int meu_set_schedule(meu_handle* h, const int32_t* in3);
 
 /* Adjoint. ---------------------------------------------------------------

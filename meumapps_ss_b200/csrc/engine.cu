@@ -626,9 +626,9 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
   }
 }
 
-// Generic path: time the radix plans and column tiles of the compile-time transforms
-// (forward and inverse of V fields, the batch of the driving-force transforms) and
-// keep the fastest.
+// Generic path: time the rule of FFT3::by_rule, then each radix plan and column tile of the
+// compile-time transforms (forward and inverse of V fields, the batch of the driving-force
+// transforms) and keep the fastest.
 template <typename R>
 void Engine<R>::tune_transforms() {
   const int nf = std::min(V, NS);
@@ -644,8 +644,12 @@ void Engine<R>::tune_transforms() {
   MEU_CUDA(cudaEventCreate(&e1));
   float best = 0;
   int best_pv = 0, best_ct = 1;
-  for (int cand = 0; cand < 4; ++cand) {
-    const int pv = (cand & 1) ? 2 : 0, ct = (cand & 2) ? 2 : 1;
+  bool best_ruled = true;
+  const bool rule = fft->by_rule(sizeof(R) == 8);  // where the rule is not plan (0, 1) itself
+  for (int cand = -1; cand < 4; ++cand) {
+    if (cand == 0 && !rule) continue;
+    const int pv = cand > 0 && (cand & 1) ? 2 : 0, ct = cand > 0 && (cand & 2) ? 2 : 1;
+    fft->ruled = cand < 0;
     fft->pv = pv;
     fft->ct = ct;
     for (int i = 0; i < 2; ++i) {
@@ -661,14 +665,16 @@ void Engine<R>::tune_transforms() {
     MEU_CUDA(cudaEventSynchronize(e1));
     float ms = 0;
     MEU_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    if (cand == 0 || ms < best) {
+    if (cand < 0 || ms < best) {
       best = ms;
+      best_ruled = fft->ruled;
       best_pv = pv;
       best_ct = ct;
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  fft->ruled = best_ruled;
   fft->pv = best_pv;
   fft->ct = best_ct;
   MEU_CUDA(cudaMemsetAsync(sp, 0, sizeof(C) * (size_t)NS * nk, st));
@@ -683,6 +689,7 @@ void Engine<R>::set_schedule(const int32_t* in3) {
     if ((in3[0] != 0 && in3[0] != 2) || in3[1] != 0 || (in3[2] != 1 && in3[2] != 2))
       throw CudaError("generic path: the schedule is (radix plan 0 or 2, 0, column-tile factor 1 or 2)",
                       MEU_ERR_UNSUPPORTED);
+    fft->ruled = false;
     fft->pv = in3[0];
     fft->ct = in3[2];
     return;

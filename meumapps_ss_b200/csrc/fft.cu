@@ -305,8 +305,8 @@ static bool cols_s(bool mix, int L, int pv, int ct, int nf, int outer, int inner
   return dispatch_len(L, pv, go) || (mix && cols_mix<R, FWD>(L, nf, outer, inner, ostride, in, out, tw, scale, st));
 }
 
-// Radix plan and column-tile factor of the power-of-two passes on the default plan (pv 0, ct 1), by
-// length, direction and precision, where by_rule() lets it choose.  The forward pass loads its
+// Radix plan and column-tile factor of the power-of-two passes by length, direction and precision,
+// where by_rule() lets it choose.  The forward pass loads its
 // first butterflies from global memory and stores through the digit reversal, the inverse the
 // other way round, and radix 16 needs twice the registers in FP64, so they do not agree.  us per
 // launch of six fields, (0, 1) / chosen: FP32 256^3 y 163 / 139 forward, 173 / 126 inverse; FP32

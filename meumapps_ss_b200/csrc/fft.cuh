@@ -342,12 +342,12 @@ class FFT3 {
   // compile-time kernels for the lengths with factors 3 (else their run-time plan, whose
   // rounding differs: see Engine::keep_rounding)
   bool mix = true;
-  // The default (pv 0, ct 1) leaves plan and tile of the y and z passes to the rule in fft.cu: in
-  // FP64, and in FP32 while `fast` is set.  An FP32 pair on radix 16 rounds about a fifth more than
+  // Unless a caller has chosen pv and ct (and cleared `ruled`), plan and tile of the y and z passes
+  // follow the rule in fft.cu: in FP64, and in FP32 while `fast` is set.  An FP32 pair on radix 16 rounds about a fifth more than
   // on radix 8 (256^3, el_en against 64 bits 9.9e-7, 8.2e-7), which the order parameters would
   // feel (el_en takes their error six times) and the iterates of the elastic fixed point do not.
-  bool fast = false;
-  bool by_rule(bool f64) const { return mix && pv == 0 && ct == 1 && (f64 || fast); }
+  bool ruled = true, fast = false;
+  bool by_rule(bool f64) const { return mix && ruled && (f64 || fast); }
   LaunchHook* hook = nullptr;
   const void* post_tw;  // cplx<R>[nx/2+1]: exp(-2 pi i k / nx)
   bool fp64;
