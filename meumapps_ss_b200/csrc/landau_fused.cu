@@ -87,6 +87,7 @@ void tune_load() {
   while (f >> prec >> N >> V >> members >> energy >> s.pv >> s.ntp >> s.tm) {
     std::string rest;
     std::getline(f, rest);
+    if (s.tm == 0) s.tm = prec == "f64" ? 8 : 16;  // a file may leave the wide tile unnamed
     g_tune[tune_key(prec == "f64", N, V, members, energy != 0)] = s;
   }
 }

@@ -32,3 +32,22 @@ def test_generic_plan_that_is_set_runs_in_every_pass():
             g.run(2)
             out.append(g.get_fields(ustate=True))
     assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+def test_saved_schedule_without_a_tile_is_the_wide_tile(tmp_path):
+    saved = tmp_path / "tuned.txt"
+    saved.write_text("f32 32 2 1 1 0 512 0 0.02\nf64 32 2 1 1 0 512 0 0.02\n")
+    code = ("from helpers import active_landau\n"
+            "from meumapps_ss_b200 import params as P\n"
+            "from meumapps_ss_b200.sim import Simulation\n"
+            "for prec, tm in ((P.PREC_F32, 16), (P.PREC_F64, 8)):\n"
+            "    p, c, e = active_landau(32, 2, precision=prec)\n"
+            "    p.flags |= P.FLAG_AUTOTUNE\n"
+            "    with Simulation(p) as g:\n"
+            "        assert g.schedule == (0, 512, tm), g.schedule\n"
+            "        g.set_fields(c, e)\n"
+            "        g.run(1)\n")
+    env = dict(os.environ, MEU_AUTOTUNE_CACHE=str(saved),
+               PYTHONPATH=os.pathsep.join([ROOT, os.path.join(ROOT, "tests"), os.environ.get("PYTHONPATH", "")]))
+    r = subprocess.run([sys.executable, "-c", code], env=env, cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
