@@ -91,17 +91,22 @@ struct LanFusedArgs {
 struct LanSched {
   int pv = 0, ntp = 512, tm = 0;  // of a handle: lan_default
 };
-// Column tile of a handle that sets none.  The column kernels are bound by latency, so more and
-// smaller blocks win until a tile's runs in global memory (tm complex) get short.  Measured on the
-// default radix plan and plane threads, us per step:
+// Column tile of a handle that sets none.  The column kernels are bound by latency, so on one grid
+// more and smaller blocks win until a tile's runs in global memory (tm complex) get short.  Where an
+// ensemble's members fill the SMs the wide tile wins instead, and members run the schedule of
+// single handles, so that their rows agree bit for bit.  The narrow tile is the default where a
+// single grid gains more than an ensemble loses (MEU_ENS_AUTOTUNE times both for an ensemble).
+// us per step, narrow / wide, on the default radix plan and plane threads:
 //  FP32 8 / 16 columns: 128^3 two variants 126 / 134, three 176 / 188, four 221 / 249; 64^3 two to
-//   four 33.9 / 40.0, 37.5 / 47.2, 44.8 / 52.8.  One variant keeps 16: a single grid gains at most
-//   9% (48^3), but the members of an ensemble fill the GPU anyway and lose 6% on average, and
-//   they run the schedule of single handles;
-//  FP64 4 / 8 columns: 32^3 two to four variants 20.6 / 21.5, 21.5 / 23.3, 23.5 / 28.1; 48^3 two to
-//   four 35.2 / 31.1, 37.9 / 44.4, 42.3 / 49.4; 64^3 and larger 8 (4 is 0 to 17% slower).
+//   four 33.9 / 40.0, 37.5 / 47.2, 44.8 / 52.8.  16 members of 64^3 276 / 250, 362 / 351, 461 / 442, of
+//   48^3 168 / 157, 229 / 210, 289 / 265, of 32^3 70 / 66, 87 / 84, 109 / 104; 8 of 128^3 798 / 817,
+//   1159 / 1188, 1469 / 1646.  One variant keeps 16: a single grid gains at most 9% (48^3),
+//   ensembles lose 6%;
+//  FP64 4 / 8 columns: 48^3 three and four variants 37.9 / 44.4, 42.3 / 49.4, 16 members 355 / 333,
+//   447 / 425; 32^3 21.5 / 23.3, 23.5 / 28.1, 16 members 121 / 104, 151 / 132.  Two variants keep 8 (32^3
+//   20.6 / 21.5, 16 members 98 / 83; 48^3 35.2 / 31.1), and so do 64^3 and larger (0 to 17% slower).
 inline int lan_default_tm(int N, int V, bool f64) {
-  if (f64) return (N <= 48 && V >= 3) || (N <= 32 && V >= 2) ? 4 : 8;
+  if (f64) return N <= 48 && V >= 3 ? 4 : 8;
   return V == 1 ? 16 : 8;
 }
 // Schedule of a handle that sets none.  The radix plan and the plane threads, us per step:

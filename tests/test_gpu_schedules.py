@@ -51,3 +51,16 @@ def test_saved_schedule_without_a_tile_is_the_wide_tile(tmp_path):
                PYTHONPATH=os.pathsep.join([ROOT, os.path.join(ROOT, "tests"), os.environ.get("PYTHONPATH", "")]))
     r = subprocess.run([sys.executable, "-c", code], env=env, cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("n,nvar,precision,tile", [(32, 2, P.PREC_F64, 8), (32, 3, P.PREC_F64, 4), (48, 2, P.PREC_F64, 8),
+                                                   (48, 3, P.PREC_F64, 4), (64, 4, P.PREC_F64, 8),
+                                                   (32, 1, P.PREC_F32, 16), (32, 2, P.PREC_F32, 8)])
+def test_default_column_tile(n, nvar, precision, tile):
+    # the narrow tile only where a single grid gains more from it than an ensemble of such grids loses
+    from meumapps_ss_b200.sim import Ensemble, Simulation
+    eig = [[0.01] * 3] if nvar == 1 else CF.tetragonal_variants(0.02, -0.005, nvar)
+    p = CF.landau_params(n, nvar, eig, precision=precision)
+    with Simulation(p) as g:
+        assert g.schedule == (0, 512, tile)
+    assert Ensemble([p, p]).schedule(1)[:3] == (0, 512, tile)
