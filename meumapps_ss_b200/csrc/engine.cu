@@ -1146,18 +1146,8 @@ void Engine<R>::kks_step(meu_diag* d) {
   }
   // local driving force (:619-845)
   {
-    // compile-time counts for the common decks (composition solve and variants in registers)
-    auto kp = k_kks_point<R>;
-    if (P.numph == 2 && P.numel == 1) {
-      kp = V == 1 ? k_kks_point<R, 2, 1, 1> : V == 3 ? k_kks_point<R, 2, 1, 3> : V == 12 ? k_kks_point<R, 2, 1, 12>
-                                                                                         : k_kks_point<R, 2, 1>;
-    } else if (P.numph == 3 && P.numel == 1) {
-      kp = k_kks_point<R, 3, 1>;
-    } else if (P.numph == 2 && P.numel == 2) {
-      kp = V == 1 ? k_kks_point<R, 2, 2, 1> : V == 3 ? k_kks_point<R, 2, 2, 3> : k_kks_point<R, 2, 2>;
-    }
     KLAUNCH("kks_point", (double)(7 * V + 4 * E) * n3 * sizeof(R),
-            kp<<<RED_BLOCKS, RED_THREADS, 0, st>>>(kks_par, phi, c, wr, pphi, fd, fc, partials, d_err));
+            kks_point_kernel<R>(P.numph, E, V)<<<RED_BLOCKS, RED_THREADS, 0, st>>>(kks_par, phi, c, wr, pphi, fd, fc, partials, d_err));
   }
   // elasticity (:851-880); on the row path elener writes the TDGL right-hand side into fd
   last_iters = 0;

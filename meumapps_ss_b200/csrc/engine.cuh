@@ -78,6 +78,11 @@ int el_z_blocks(int nz, int inner);
 // sp: six contiguous spectra; part: [6][el_z_blocks] partial sums of the convergence test
 template <typename R>
 void el_z_launch(const FFT3& f, cplx<R>* sp, cplx<R>* uk, const ElzCoef& E, double* part, cudaStream_t st);
+// driving force of the KKS step (k_kks_point) for the deck's counts (kks_point.cuh)
+template <typename R>
+using KksPointFn = void (*)(KksPar, const R*, const R*, const R*, R*, R*, R*, double*, int*);
+template <typename R>
+KksPointFn<R> kks_point_kernel(int numph, int numel, int nvar);
 // derivatives along one axis (deriv.cuh): field v of the launch at f + v * fs;
 // out = base + s (acc + D f), lap (+)= g D2 f (NULL: not formed)
 template <typename R>

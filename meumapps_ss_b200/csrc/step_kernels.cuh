@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) k_kks_lap(const DevConst* __restrict__ Kp
 // Fields in R; the local solve and the energies in FP64.  NPH, NEL > 0: the phase and solute
 // counts are compile-time (the common decks), so the zdim x zdim composition system and its
 // inverse live in registers; NV > 0: the variant count too, so the per-variant values do and the
-// voxel's loads are all in flight together (KKS 128^3, 3 variants: 231 -> 125 us).  0: any counts,
+// voxel's loads are all in flight together (KKS 128^3, 3 variants: 231 -> 90 us).  0: any counts,
 // arrays sized for the largest system (local memory).
 template <typename R, int NPH = 0, int NEL = 0, int NV = 0>
 __global__ void __launch_bounds__(RED_THREADS, NV > 0 && NV <= 4 ? 2 : 1)
