@@ -540,9 +540,9 @@ Engine<R>::Engine(const meu_params& p) : P(p) {
       for (int i = 0; i < 6; ++i)
         for (int j = 0; j < i; ++j) sym = sym && hK.c0m[i + j * 6] == hK.c0m[j + i * 6];
       elz_blocks = sym ? el_z_blocks<R>(p.nz, p.ny * hK.nxh) : 0;
-      // (its plan and scaling are the separate passes' where nz is 32 or 64 and the cell count a
-      // power of two)
-      if (keep_rounding && !((p.nz == 32 || p.nz == 64) && (n3 & (n3 - 1)) == 0)) elz_blocks = 0;
+      // where rounding is kept, only if its radix plan is that of the separate compile-time passes
+      // (powers of two from 32 on; 32, 64 and 512 have it) and scaling by 1 / n3 is exact
+      if (keep_rounding && !(p.nz >= 32 && fz::same_plan(p.nz, 3, 0) && (n3 & (n3 - 1)) == 0)) elz_blocks = 0;
       if (elz_blocks) {
         elz_part = dalloc<double>(6 * (int64_t)elz_blocks);
         int ex = 0;
@@ -1006,6 +1006,8 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
   };
   if (!zeroth_only) {
     FastPasses fast_passes(*fft);
+    // a plan that the caller set is the z passes' too where rounding is kept
+    const bool z_fused = elz_blocks > 0 && (!keep_rounding || fft->pv == 0);
     // The control runs on the device.  An iteration before the el_min_iter'th cannot end the
     // loop, so those are queued together: one wait of the host per step instead of one per
     // iteration where el_min_iter suffice.
@@ -1038,7 +1040,7 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
         // ---- y, k-space, y
         const ElCtlArgs ca{d_ctl, P.el_tol, (double)n3, P.el_min_iter, P.el_max_iter, total == 1 ? 1 : 0};
         fft->pass_y<R>(S6, 6, true, st);
-        if (elz_blocks) {
+        if (z_fused) {
           if (!elz_q_checked && i == 0) KLAUNCH("el_qcheck", 0.0, k_el_qcheck<<<gridk(), 256, 0, st>>>(dK, d_err));
           KLAUNCH("el_z", 18.0 * nk * sizeof(C), el_z_launch<R>(*fft, S6.p[0], uk, elz, elz_part, st));
           KLAUNCH("finalize", 48.0 * elz_blocks,
@@ -1060,7 +1062,7 @@ void Engine<R>::elastic(const R* ph_for_ppr, R* elg, const EnerOut<R>& eo, bool 
       MEU_CUDA(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(ElCtl), cudaMemcpyDeviceToHost, st));
       MEU_CUDA(cudaStreamSynchronize(st));
       if (h_ctl->err) raise_err(h_ctl->err);
-      elz_q_checked = elz_blocks > 0;
+      elz_q_checked = elz_q_checked || z_fused;
       if (h_ctl->status) throw CudaError("newfac is too small ... trouble converging", h_ctl->status);
       if (h_ctl->done) break;
     }

@@ -64,3 +64,31 @@ def test_default_column_tile(n, nvar, precision, tile):
     with Simulation(p) as g:
         assert g.schedule == (0, 512, tile)
     assert Ensemble([p, p]).schedule(1)[:3] == (0, 512, tile)
+
+
+@pytest.mark.parametrize("nz,pv,fused_z", [(32, 0, True), (64, 0, True), (512, 0, True), (64, 2, False), (128, 0, False),
+                                           (16, 0, False)])
+def test_fp32_variants_keep_the_rounding_of_their_z_plan(nz, pv, fused_z):
+    # FP32 decks of several variants run the fused z kernel only where its radix plan is the one that
+    # the separate passes would run; the plan that a caller sets is kept either way
+    from meumapps_ss_b200.sim import Simulation
+    _, p, cons, phi = kks_case(16, 3, 4, ny=8, nz=nz)
+    rng = np.random.default_rng(nz)
+    # every variant present everywhere: n_tilda counts signs that rounding does not decide
+    phi = np.clip(phi + rng.uniform(0.1, 0.3, phi.shape), 0.0, 1.0)
+    out = {}
+    for prec in (P.PREC_F64, P.PREC_F32):
+        q = p.copy()
+        q.precision = prec
+        with Simulation(q) as g:
+            if pv:
+                g.set_schedule(pv, 0, 1)
+            g.set_fields(cons, phi)
+            g.timing(True)
+            g.run(2)
+            names = set(g.timing_report())
+            out[prec] = g.get_fields()
+        assert ("el_z" in names) == (fused_z or prec == P.PREC_F64), names
+    # FP32 fields: 64 roundings bound two steps
+    for a, b in zip(out[P.PREC_F32][:2], out[P.PREC_F64][:2]):
+        assert np.linalg.norm(a - b) <= 64 * 2.0 ** -24 * np.linalg.norm(b)
