@@ -57,7 +57,8 @@ struct CudaError : std::runtime_error {
 // first statement, until that kernel has completed and its writes are visible.  The release comes
 // after the wait, so when a chained kernel is placed, everything before its predecessor is
 // complete.  Such kernels read what another kernel writes through pointers without __restrict__:
-// a read-only load must not move above the wait (or guard such loads by the bound of a loop).
+// the read-only path asks for data that nothing writes while the kernel is resident, and its loads
+// must not move above the wait.
 // KKS 48 x 36 x 54, two solutes, 20 steps: 6.27 -> 5.32 ms, 108 x 144 x 96 FP64 6.92 -> 6.52.
 // k_kks_point and k_el_ener are launched as usual: chained they cost the 128^3 KKS step 50 and
 // 20 us of its 2 ms, and gained nothing elsewhere.

@@ -968,9 +968,9 @@ __global__ void __launch_bounds__(256) k_lan_b(const DevConst* __restrict__ Kp, 
 // Multi_MEUMAPPS.f:1008-1043: clip phi (KKS), min/max C (initial 1.0 / 0.0),
 // max phi (initial 0.0), solid fraction (sum of phi>0; Landau: sum eta^2), sum C.
 template <typename R>
-__global__ void __launch_bounds__(RED_THREADS) k_stats(const DevConst* __restrict__ Kp, const R* __restrict__ c,
+__global__ void __launch_bounds__(RED_THREADS) k_stats(const DevConst* __restrict__ Kp, const R* c,
                                                        R* __restrict__ phi, int clip, double* partials) {
-  dep_enter();  // every field read below is guarded by the loop's bound
+  dep_enter();
   const DevConst& K = *Kp;
   const int64_t n3 = K.n3;
   const int V = K.p.nvar, E = K.p.numel;
