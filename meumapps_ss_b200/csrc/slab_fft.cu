@@ -85,11 +85,15 @@ void planes_forward(meu_slab_fft* h, const void* real, void* send, cudaStream_t 
   PtrList<const R> a{};
   PtrList<C> b{};
   a.p[0] = (const R*)real;
-  // one rank: the send buffer is the planes' spectrum (P = 1 packs nothing), transformed in it
-  b.p[0] = (C*)(h->P == 1 ? send : h->spec);
+  // one rank: the send buffer is the planes' spectrum (P = 1 packs nothing), transformed in it,
+  // unless it overlaps the real slab, which the x pass then still reads
+  const size_t nr = sizeof(R) * (size_t)h->nx * h->ny * h->nzl, ns = sizeof(C) * (size_t)h->nxh * h->ny * h->nzl;
+  const char *r0 = (const char*)real, *s0 = (const char*)send;
+  const bool direct = h->P == 1 && (r0 + nr <= s0 || s0 + ns <= r0);
+  b.p[0] = (C*)(direct ? send : h->spec);
   h->planes->forward_x<R>(a, b, 1, st);
   h->planes->pass_y<R>(b, 1, true, st);
-  if (h->P == 1) {
+  if (direct) {
     h->launches += 2;
     return;
   }
