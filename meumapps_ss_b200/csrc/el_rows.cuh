@@ -34,8 +34,9 @@ constexpr int PV = 4;
 //   0.38 ms; 24 KB x 256 x 3 0.41, 48 KB x 384 x 2 0.43);
 //  FP64: 24 KB, 128 threads, four blocks (KKS 128^3 0.111 ms, 24 KB x 256 x 2 0.138; 108 x 144 x 96
 //   70 us, 48 KB x 256 x 2 74 us);
-//  FP32 with general moduli (FP64 voxel work, order parameters of up to 16 variants beside the
-//   lines): 48 KB, 256 threads, two blocks (KKS 64^3, 12 variants: 25 us, 24 KB x 128 x 4 31 us).
+//  FP32 with general moduli (FP64 voxel work): 48 KB, 256 threads, two blocks.  Against 24 KB x 128 x 4
+//   small grids and many variants gain and large ones lose (KKS 64^3, one variant 16.8 us, 20.9 with the
+//   latter; Landau 64^3, 12 variants 23.4, 29.6; 128 x 128 x 64, 12 variants 73, 80; four 50.8, 46.7).
 template <typename R, bool GEN>
 struct Cfg {
   static constexpr int KB = sizeof(R) == 8 ? 24 : GEN ? 48 : 16;
